@@ -1,23 +1,33 @@
-// Prefill attention on 5th-generation tensor cores (tcgen05 + TMEM) for head_dim 128 (sm_100a).
+// Prompt attention on 5th-generation tensor cores (tcgen05 + TMEM) for head_dim 128 (sm_100a).
 //
-// Covers chatglm.cpp:655-717 for a prompt (n_past == 0, qlen = S tokens) in two launches:
-//   prefill_prepare_kernel  RoPE on q and k (:655-656), f16 append of the K rows and V^T columns (:668-675),
-//                           q * 1/sqrt(d) (:686) written as an f16 [head][token][d] tile source;
-//   prefill_attn_kernel     one CTA per (128-token q tile, q head): flash-attention forward over the freshly
-//                           written cache.  S = Q K^T (128x128x128) and O_tile = P V (128x128x128) are tcgen05.mma
-//                           instructions issued by one thread of a control warp, operands staged in shared memory by
-//                           TMA (K and V^T tiles, non-multicast, 128-byte swizzle, double buffered) or by the softmax
-//                           threads (P, double buffered), accumulators in tensor memory (two S buffers and the
-//                           running O), read back with tcgen05.ld: each of the 128 softmax threads owns one q row,
-//                           so the online softmax needs no cross-thread reduction.  O stays in tensor memory across
-//                           KV tiles (the MMA accumulates into it); a row's O is rescaled there only when its running
-//                           maximum grows by more than 2^8, otherwise the old reference maximum is kept (exact: the
-//                           same reference enters the numerator and the denominator).  The control thread runs
-//                           ahead: S of tile j+1 and P V of tile j execute while the softmax threads work on tile j+1.
-// Masks (chatglm.cpp:689-707): causal (token t visible to row s iff t <= n_virtual + s; tiles right of the
-// diagonal are skipped) or the ChatGLM-6B v1 prefix mask (every row but the last is blocked from the last token).
-// Tokens past the attended length never reach shared memory: the per-call tensor maps end at that length, so TMA
-// fills them with zeros.
+// Covers chatglm.cpp:655-717 for the sequences of a call that bring more than one token, in two launches for up to
+// kPrefillMaxSeq of them:
+//   prefill_append_kernel  RoPE on k (:655-656) and the f16 append of the K rows and V^T columns (:668-675);
+//   prefill_attn_kernel    RoPE on q, q * 1/sqrt(d) (:686) and flash attention over the cache (:687-717).
+// An attention CTA works on TWO 128-row q tiles at a time that read the same K and V^T tiles: the same token rows of two
+// q heads of one kv head, or (one q head per kv head) two neighbouring row tiles of a head.  Per 64 tokens (a step) and q tile
+// the tensor core has 640 cycles to do (Q K^T: 8 MMAs of 48 cycles, bound by the shared-memory reads of both operands; P V: 4 of
+// 64) and the exponential unit 512 (16 per cycle): with one q tile in flight the two alternate, with two they overlap.
+//   softmax warps  two groups of four; a thread owns one q row of its group's tile (one tensor-memory lane), so the online
+//                  softmax needs no cross-thread reduction.  The scores of a step are released as soon as they are in
+//                  registers; the probabilities go back to TENSOR memory and are the A operand of P V there: no shared
+//                  memory, no proxy fence.
+//   load warp      TMA: K and V^T tiles alternate through one ring (non-multicast, 128-byte swizzle).
+//   MMA warps      one per group.  Q K^T of step t + 1 runs while the softmax works on step t, P V of t follows it.  tcgen05.mma
+//                  of one thread execute in order: a group that sees its scores of step t knows that P V of t - 2 has landed.
+//   q warps        stage the q tiles of the CTA's next unit (CTAs are persistent; units are dealt longest first).
+// Measured (B200, 32 q heads, 2 kv heads, causal, f16 activations): an 8192-token prompt alone 499 us, 563 us back to back
+// under the power cap (977 TFLOP/s of useful work), against 795 us with one q tile per CTA, probabilities through shared memory and q staged through HBM by a kernel of its own.
+// A step takes about 1600 cycles; taking a quarter of the exponentials off their unit (a polynomial on the FMA pipe) made it
+// slower, because what the softmax warps issue delays the MMA warps, which need about a tenth of the issue slots.
+// O stays in tensor memory across KV tiles; a row's O is rescaled there only when its running maximum grows by more than
+// 2^8, otherwise the old reference maximum is kept (exact: the same reference enters numerator and denominator).
+// Masks (chatglm.cpp:689-707, at n_past == 0 only): causal (token t visible to row s iff t <= n_virtual + s; tiles right
+// of the diagonal are skipped) or the ChatGLM-6B v1 prefix mask (every row but the last is blocked from the last token).
+// Tokens past the attended length: their scores are masked whatever the cache holds there, and the V^T tensor map of a
+// sequence ends at its attended length, so TMA fills the rest with zeros.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace cglm {
@@ -25,102 +35,209 @@ namespace cglm {
 namespace {
 
 constexpr int kD = 128;
-constexpr int kQTile = 128;        // q rows per CTA = TMEM lanes
-constexpr int kKvTile = 128;       // tokens per KV tile
-constexpr int kSoftmaxThreads = 128;
-constexpr int kLoadWarp = kSoftmaxThreads / 32;       // issues every TMA load
-constexpr int kScoreWarp = kLoadWarp + 1;             // issues the S = Q K^T MMAs
-constexpr int kPvWarp = kLoadWarp + 2;                // issues the O += P V MMAs
-constexpr int kThreads = kSoftmaxThreads + 96;
-constexpr int kHalfBytes = 128 * 128;          // one 128-row x 128-byte swizzled half tile (16 KiB)
-constexpr int kTileBytes = 2 * kHalfBytes;     // a 128 x 128 f16 operand tile
-constexpr int kTmemCols = 512;                 // S[2]: columns [0,256), O: columns [256,384)
-constexpr float kRescaleThreshold = 8.f;       // log2 units a row's maximum may grow before O is rescaled
-constexpr int kOutStride = 132;                // floats per row of the output staging tile
+constexpr int kQTile = 128;                   // q rows per tile = TMEM lanes
+constexpr int kKvTile = 128;                  // tokens per TMA tile of K or V^T
+constexpr int kStep = 64;                     // tokens per softmax step: half a tile
+constexpr int kGroupThreads = 128;            // softmax threads per q tile
+constexpr int kQWarp = 8;                     // four warps that stage the q tiles of a CTA's next unit
+constexpr int kLoadWarp = 12;                 // issues the TMA loads of K and V^T
+constexpr int kMmaWarp = 13;                  // kMmaWarp + w issues the MMAs of group w
+constexpr int kThreads = 16 * 32;             // (warp 15 idle: register shares are handed out per four warps)
+constexpr int kSoftmaxRegs = 168, kOtherRegs = 88;   // 256 x 168 + 256 x 88 = the 65536 registers the CTA is launched with
+constexpr int kHalfBytes = 128 * 128;         // one 128-row x 128-byte swizzled half tile (16 KiB)
+constexpr int kTileBytes = 2 * kHalfBytes;    // a 128 x 128 f16 operand tile
+constexpr int kStages = 5;                    // ring of K and V^T tiles: K(0), V(0), K(1), V(1), ...
+constexpr int kTmemCols = 512;                // group w: S at columns 128 w, P buffers at 128 w + 64 and + 96, O at 256 + 128 w
+constexpr float kRescaleThreshold = 8.f;      // log2 units a row's maximum may grow before O is rescaled
 constexpr float kLog2e = 1.4426950408889634f;
 
-// instruction descriptor of tcgen05.mma.kind::f16: D = f32, A = B = f16, both K-major, N = 128, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+// instruction descriptors of tcgen05.mma.kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = 64 (scores) / 128 (P V)
+constexpr uint32_t kIdescS = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+constexpr uint32_t kIdescO = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
 struct __align__(1024) PrefillSmem {
-    uint8_t q[kTileBytes];            // A of QK^T: [2 d-halves][128 rows][64 d]
-    uint8_t k[2][kTileBytes];         // B of QK^T: [2 d-halves][128 tokens][64 d], double buffered
-    uint8_t v[2][kTileBytes];         // B of PV:   [2 token-halves][128 d][64 tokens], double buffered
-    uint8_t p[2][kTileBytes];         // A of PV:   [2 token-halves][128 rows][64 tokens], double buffered
-    uint64_t q_full;
-    uint64_t k_full[2];               // TMA -> control: K tile landed
-    uint64_t v_full[2];               // TMA -> control: V^T tile landed
-    uint64_t s_done[2];               // tensor core -> softmax: S buffer written
-    uint64_t p_ready[2];              // softmax -> control: P buffer written, S buffer read
-    uint64_t o_done[2];               // tensor core -> softmax, control: P V(j) accumulated; K/V^T[b] and P[b] have been read
+    uint8_t q[2][kTileBytes];         // A of QK^T per group: [2 d-halves][128 rows][64 d]; staging of the output at the end
+    uint8_t kv[kStages][kTileBytes];  // K tile [2 d-halves][128 tokens][64 d] or V^T tile [2 token-halves][128 d][64 tokens]
+    uint64_t kv_full[kStages];        // TMA -> MMA: tile landed
+    uint64_t kv_empty[kStages];       // tensor core -> TMA: tile has been read by both groups' MMAs
+    uint64_t q_full[2];               // q tile of a unit in place (first unit: softmax group, later ones: bulk copy) -> MMA
+    uint64_t q_empty[2];              // tensor core -> q warps: the unit's last scores computed
+    uint64_t s_full[2];               // tensor core -> softmax group: scores of a step written
+    uint64_t s_empty[2];              // softmax group -> MMA: scores are in registers
+    uint64_t p_full[2][2];            // softmax group -> MMA: probabilities of a step written, O rescaled if it had to be (per buffer)
+    uint64_t o_step[2];               // tensor core -> softmax group: P V of a step accumulated (looked at before a rescale)
+    uint64_t o_full[2];               // tensor core -> softmax group: the unit's last P V accumulated
+    uint64_t o_empty[2];              // softmax group -> MMA: O of the unit has been read
     uint32_t tmem_base;
     int abort_flag;
 };
 static_assert(sizeof(PrefillSmem) + 1024 <= 232448, "one prefill CTA must fit the shared memory of an SM");
-static_assert(kTileBytes * 4 >= 128 * kOutStride * 4, "the K/V^T buffers hold the output staging tile");
 
-// shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-    return static_cast<uint64_t>((saddr & 0x3ffffu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 bytes apart.  Its upper word is the
+// same for every operand here; an operand `bytes` further on has the lower word + (bytes >> 4).
+constexpr uint32_t kDescHi = 64u | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr & 0x3ffffu) >> 4) | (1u << 16); }
+// MMAs and commits of a warp: every lane runs through them and `lead` (one lane's 1) predicates the instruction itself, so that
+// the operands are computed in uniform registers; behind a branch on the elected lane each of them was moved there one by one,
+// and issuing a 48-cycle MMA took longer than that while the softmax warps kept the schedulers busy.
+template <uint32_t kIdesc, bool kAccumulate>
+__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t lead) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdesc), "r"(accumulate), "r"(0u)
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 ad, bd;\n\tmov.b64 ad, {%1, %5};\n\tmov.b64 bd, {%2, %5};\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], ad, bd, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kIdesc), "n"(kAccumulate ? 1 : 0), "r"(kDescHi), "r"(lead)
         : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
+// A from tensor memory: lane = row, one 32-bit column = two consecutive k
+template <uint32_t kIdesc>
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t accumulate, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 bd;\n\tmov.b64 bd, {%2, %5};\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(kIdesc), "r"(accumulate), "r"(kDescHi), "r"(lead)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint64_t *bar, uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        ::"r"(smem_u32(bar)), "r"(lead)
+        : "memory");
+}
+// 1 in one lane of the (converged) warp
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t pred;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+    return pred;
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// packed f32x2 arithmetic and the three-input maximum of sm_100: half the instructions of the scalar forms
-__device__ __forceinline__ void fma2(float &d0, float &d1, float a0, float a1, float b, float c) {
-    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %4};\n\tmov.b64 rc, {%5, %5};\n\t"
-        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-        : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "f"(b), "f"(c));
-}
-__device__ __forceinline__ void add2(float &d0, float &d1, float a0, float a1) {   // (d0, d1) += (a0, a1)
-    asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%0, %1};\n\tmov.b64 rb, {%2, %3};\n\tadd.rn.f32x2 rd, ra, rb;\n\t"
-        "mov.b64 {%0, %1}, rd;\n\t}"
-        : "+f"(d0), "+f"(d1) : "f"(a0), "f"(a1));
-}
+// the three-input maximum of sm_100
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-// 32 consecutive f32 columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-    uint32_t r[32];
+// 32 consecutive f32 columns of this thread's TMEM lane, without the wait
+__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t *r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
           "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
         : "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
 }
 
-// ---- launch 1: RoPE, append, f16 q ---------------------------------------------------------------------------
-// Grid: (16-token blocks, roles).  Roles along y: pairs of q heads, then one CTA per k head, then one CTA per v head.
-//   q / k CTAs  rotate their heads for the block's tokens with cos/sin from the arena's angle table (or, for
-//               caller-supplied position ids, from a table rope_table_kernel filled just before);
-//   v CTAs      transpose [16 tokens][128 dims] through shared memory so that the V^T cache rows are written as
-//               contiguous runs of tokens instead of one 2-byte store per (token, dim).
-// q_half: f16 [H][s_pad][D]; rows >= S are never read for an output.  Rope modes: the two GLM modes or none.
-static int rope_n_pairs_host(int rope_type) { return rope_type == CGLM_ROPE_DISABLED ? 0 : 1; }
-constexpr int kPrepTokens = 16;   // tokens per CTA: one batch of loads per thread (64 measured 2.4 us slower per call)
-constexpr int kPrepThreads = 256;
+// ---- q and k rows: half a warp per 128-element row, lane hl of it owning dims 8 hl .. 8 hl + 7 -----------------------------------
+// Loading, rotating and storing are separate, so that a warp has several rows of loads in flight; everything is kept small,
+// because a CTA runs this code once, out of a cold instruction cache (a version with a quarter of a row per lane and eight rows
+// unrolled took 8 us for 57 tokens).
+struct Row8 {
+    uint4 r[2];    // raw activations: eight f32, or eight f16 in r[0]
+    float4 a[4];   // (cos, sin) pairs: CHATGLM2 two float4 (four pairs), CHATGLM four (eight)
+};
+// Row s of a tensor whose head starts at element e_head.  s >= n_tok: zeros.  vec: rows are 16-byte (f32) or 8-byte (f16) aligned.
+__device__ __forceinline__ void load_row8(Row8 &x, const PrefillSeq &ps, int rope_type, const float *base, long long e_head, long long stride,
+                                          int s, int hl) {
+    const SeqDev &sq = ps.sq;
+    const bool f16 = (sq.flags & CGLM_SEQ_QKV_F16) != 0;
+    x.r[0] = x.r[1] = make_uint4(0u, 0u, 0u, 0u);
+    const long long e = e_head + s * stride + 8 * hl;
+    if (s < sq.qlen) {
+        if (ps.vec && f16) {
+            const uint2 *p = reinterpret_cast<const uint2 *>(reinterpret_cast<const __half *>(base) + e);
+            const uint2 u = __ldg(p), v = __ldg(p + 1);
+            x.r[0] = make_uint4(u.x, u.y, v.x, v.y);
+        } else if (ps.vec) {
+            const uint4 *p = reinterpret_cast<const uint4 *>(base + e);
+            x.r[0] = __ldg(p);
+            x.r[1] = __ldg(p + 1);
+        } else if (f16) {
+            const unsigned short *p = reinterpret_cast<const unsigned short *>(base) + e;
+            x.r[0] = make_uint4(p[0] | p[1] << 16, p[2] | p[3] << 16, p[4] | p[5] << 16, p[6] | p[7] << 16);
+        } else {
+            const uint32_t *p = reinterpret_cast<const uint32_t *>(base) + e;
+            x.r[0] = make_uint4(p[0], p[1], p[2], p[3]);
+            x.r[1] = make_uint4(p[4], p[5], p[6], p[7]);
+        }
+    }
+    // Angles: by_position: the arena's table, indexed by the derived ids (chatglm.cpp:1142-1153, 1319-1327); otherwise the table
+    // rope_table_kernel filled for this call, [stream][token].
+    const int sc = min(s, sq.qlen - 1);
+    if (rope_type == CGLM_ROPE_CHATGLM2) {           // dims [0, 64) as adjacent pairs: lanes 0..7, ladder steps 4 hl .. 4 hl + 3
+        const int row = ps.by_position ? sq.n_past + sc : sc;
+        const float4 *t = reinterpret_cast<const float4 *>(ps.angles + static_cast<long long>(row) * 32 + 4 * (hl & 7));
+        x.a[0] = __ldg(t);
+        x.a[1] = __ldg(t + 1);
+    } else if (rope_type == CGLM_ROPE_CHATGLM) {     // each 64-dim half as pairs (i, i + 32): ladder steps 8 (hl & 3) .. + 7
+        const bool second = hl >= 8;                 // by the position id, the second half by the block position id
+        const int p = sq.n_past + sc, lim = sq.n_ctx - 2;
+        const int row = ps.by_position ? (second ? max(p - lim, 0) : min(p, lim)) : (second ? sq.qlen + sc : sc);
+        const float4 *t = reinterpret_cast<const float4 *>(ps.angles + static_cast<long long>(row) * 32 + 8 * (hl & 3));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x.a[i] = __ldg(t + i);
+    }
+}
+// The rotated row.  Every product and sum rounded separately, in the order of rope_rotate().
+__device__ __forceinline__ void rotate_row8(const Row8 &x, bool f16, int rope_type, int hl, float (&y)[8]) {
+    const uint32_t w[8] = {x.r[0].x, x.r[0].y, x.r[0].z, x.r[0].w, x.r[1].x, x.r[1].y, x.r[1].z, x.r[1].w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&w[i]));
+        y[2 * i] = h.x;
+        y[2 * i + 1] = h.y;
+    }
+    if (!f16) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(w[i]);
+    }
+    if (rope_type == CGLM_ROPE_CHATGLM2) {
+        const float4 a[2] = {x.a[0], x.a[1]};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float c = i & 1 ? a[i >> 1].z : a[i >> 1].x, s = i & 1 ? a[i >> 1].w : a[i >> 1].y;
+            float y0, y1;
+            rope_rotate(y[2 * i], y[2 * i + 1], c, s, y0, y1);
+            if (hl < 8) { y[2 * i] = y0; y[2 * i + 1] = y1; }
+        }
+    } else if (rope_type == CGLM_ROPE_CHATGLM) {
+        const bool upper = (hl & 4) != 0;   // holds x_{i + 32}; the pair's other element sits four lanes away
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float c = i & 1 ? x.a[i >> 1].z : x.a[i >> 1].x, s = i & 1 ? x.a[i >> 1].w : x.a[i >> 1].y;
+            const float o = __shfl_xor_sync(0xffffffffu, y[i], 4);
+            const float p = __fmul_rn(o, s), q = __fmul_rn(y[i], c);
+            y[i] = upper ? __fadd_rn(p, q) : __fsub_rn(q, p);   // x_i: x c - o s; x_{i + 32}: o s + x c
+        }
+    }
+}
+__device__ __forceinline__ uint4 pack_half8(const float (&y)[8]) {
+    return make_uint4(pack_half2(y[0], y[1]), pack_half2(y[2], y[3]), pack_half2(y[4], y[5]), pack_half2(y[6], y[7]));
+}
+__device__ __forceinline__ void st_f32x8(float *p, const float (&y)[8]) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        reinterpret_cast<float4 *>(p)[0] = make_float4(y[0], y[1], y[2], y[3]);
+        reinterpret_cast<float4 *>(p)[1] = make_float4(y[4], y[5], y[6], y[7]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p[i] = y[i];
+    }
+}
 
-// table: f32 [stream][token][32 ladder steps][cos, sin]
+// table: f32 [stream][token][32 ladder steps][cos, sin]: only for explicit position ids, or an arena without a table
 __global__ void __launch_bounds__(256)
 rope_table_kernel(AttnShape sh, SeqDev sq, float2 *__restrict__ table) {
     const int S = sq.qlen;
@@ -135,183 +252,238 @@ rope_table_kernel(AttnShape sh, SeqDev sq, float2 *__restrict__ table) {
     table[i] = make_float2(c, s);
 }
 
-__global__ void __launch_bounds__(kPrepThreads)
-prefill_prepare_kernel(AttnShape sh, SeqDev sq, uint16_t *__restrict__ k_base, uint16_t *__restrict__ v_base,
-                       __half *__restrict__ q_half, int s_pad, const float2 *__restrict__ table, int table_by_position) {
-    // Launched as a programmatic dependent itself (its launch latency hides behind the previous kernel of the
-    // stream): nothing is read or written before that kernel has completed.  The attention kernel that follows is a
-    // programmatic dependent of this grid: let its CTAs take their places (shared memory, tensor memory, barriers)
-    // while this grid runs; it waits for this grid before its first load.
+// ---- launch 1: RoPE on k, append of K rows and V^T columns -----------------------------------------------------------------
+// Grid: (64-token blocks of all sequences, kv heads, {K, V}).
+//   K CTAs  half a warp per token row, eight rows of loads in flight per warp;
+//   V CTAs  transpose [64 tokens][128 dims] through shared memory, so that a V^T cache row is written as 128 contiguous
+//           bytes (16 per thread when the append position is a multiple of 8 tokens).
+// Bound by latency for two kv heads (a few MB), by HBM for the 32 of ChatGLM-6B.  The q rows do not pass through here (staging
+// them as f16 took 99 of the 810 us of an 8192-token prompt): the attention kernel rotates them on their way to shared memory.
+constexpr int kAppTokens = 64;
+constexpr int kAppThreads = 256;
+
+__global__ void __launch_bounds__(kAppThreads)
+prefill_append_kernel(const __grid_constant__ PrefillTable tab, AttnShape sh, uint16_t *__restrict__ k_base, uint16_t *__restrict__ v_base) {
+    // Launched as a programmatic dependent: nothing is read or written before the previous kernel of the stream has
+    // completed.  The attention kernel that follows may take its place as soon as every CTA here has passed that wait: its q
+    // rows are then final, and it waits for this grid before it reads the cache.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ __half tile_mem[kD][kPrepTokens + 2];       // v CTAs: [dim][token] transpose tile
-    const int S = sq.qlen, H = sh.H, G = sh.G, M = sh.M;
-    const bool in_f16 = (sq.flags & CGLM_SEQ_QKV_F16) != 0;
-    const int t_begin = blockIdx.x * kPrepTokens;
-    const int n_tok = min(kPrepTokens, S - t_begin);
-    const int n_qpair = (H + 1) / 2;
-    const int role = blockIdx.y;
-    const int tid = threadIdx.x;
-
-    if (role >= n_qpair + G) {
-        // ---- v head g: transpose through shared memory ---------------------------------------------------------
-        const int g = role - n_qpair - G;
-        __half(*tile)[kPrepTokens + 2] = tile_mem;
-        for (int t0 = tid >> 7; t0 < n_tok; t0 += 16) {   // 2 tokens per sweep, 8 sweeps of loads in flight
-            const int d = tid & 127;
-            float x[8];
+    // V^T tile: dim d's 64 tokens as eight 16-byte chunks, chunk c at place c ^ (d / 4 & 7): no bank conflicts either way
+    __shared__ uint4 tile[kD][kAppTokens / 8];
+    int si = 0;
+    while (si + 1 < tab.n_seq && static_cast<int>(blockIdx.x) >= tab.seqs[si + 1].block_begin) ++si;
+    const PrefillSeq &ps = tab.seqs[si];
+    const SeqDev &sq = ps.sq;
+    const int G = sh.G, M = sh.M, g = blockIdx.y;
+    const int t_begin = (static_cast<int>(blockIdx.x) - ps.block_begin) * kAppTokens;
+    const int n_tok = min(kAppTokens, sq.qlen - t_begin);
+    const bool in_f16 = (sq.flags & CGLM_SEQ_QKV_F16) != 0, vec = ps.vec != 0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long row = static_cast<long long>(sq.slot) * G + g;
+    constexpr int kRows = kAppTokens / (kAppThreads / 32);   // token rows per warp
+    if (blockIdx.z == 0) {
+        const int hl = lane & 15;
+        Row8 x[kRows / 2];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = t0 + 2 * u;
-                x[u] = t < n_tok ? ld_act(sq.v, (t_begin + t) * sq.kv_tok_stride + g * sq.kv_head_stride + d, in_f16) : 0.f;
-            }
+        for (int u = 0; u < kRows / 2; ++u)
+            load_row8(x[u], ps, sh.rope_type, sq.k, g * sq.kv_head_stride, sq.kv_tok_stride, t_begin + warp * kRows + 2 * u + (lane >> 4), hl);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = t0 + 2 * u;
-                if (t < n_tok) tile[d][t] = __float2half_rn(x[u]);
+        for (int u = 0; u < kRows / 2; ++u) {
+            const int s = t_begin + warp * kRows + 2 * u + (lane >> 4);
+            float y[8];
+            rotate_row8(x[u], in_f16, sh.rope_type, hl, y);
+            if (s < sq.qlen) {
+                *reinterpret_cast<uint4 *>(k_base + (row * M + sq.kv_before + s) * kD + 8 * hl) = pack_half8(y);
+                if (sq.k_roped) st_f32x8(sq.k_roped + (static_cast<long long>(s) * G + g) * kD + 8 * hl, y);
             }
-        }
-        __syncthreads();
-        uint16_t *vrow0 = v_base + static_cast<long long>(sq.slot * G + g) * kD * M + sq.kv_before + t_begin;
-        for (int idx = tid; idx < kD * kPrepTokens; idx += kPrepThreads) {
-            const int d = idx / kPrepTokens, t = idx % kPrepTokens;
-            if (t < n_tok) vrow0[static_cast<long long>(d) * M + t] = __half_as_ushort(tile[d][t]);
         }
         return;
     }
-
-    const int n_pairs = rope_n_pairs(sh.rope_type, kD);   // 0, 32 (CHATGLM2) or 64 (CHATGLM)
-
-    const bool is_q = role < n_qpair;
-    const int head0 = is_q ? 2 * role : role - n_qpair;
-    const int n_heads = is_q ? min(2, H - head0) : 1;
-    // p (the pair inside the head) is the same for every item of a thread: 256 threads cover 4 (token, head) rows
-    // of 64 pairs per sweep.  Loads of kBatch sweeps are issued together so that their latencies overlap.
-    const int p = tid & 63;
-    int i0, i1, cs_stream = 0, cs_ladder = 0;
-    const bool rotated = p < n_pairs;
-    if (rotated) {
-        const RopePair rp = rope_pair(sh.rope_type, kD, p);
-        i0 = rp.i0; i1 = rp.i1; cs_stream = rp.stream; cs_ladder = rp.ladder;
-    } else {
-        const int first_free = sh.rope_type == CGLM_ROPE_CHATGLM2 ? kD / 2 : 0;
-        i0 = first_free + 2 * (p - n_pairs); i1 = i0 + 1;
-    }
-    constexpr int kBatch = 8;
-    const bool v1 = sh.rope_type == CGLM_ROPE_CHATGLM;
-    const int v1_lim = sq.n_ctx - 2;
-    // table_by_position: the arena's table, row = position (or block position) of the token; otherwise the table
-    // rope_table_kernel wrote for this call, row = (stream, token)
-    const float2 *tab = table_by_position ? table + cs_ladder : table + (static_cast<long long>(cs_stream) * S + t_begin) * 32 + cs_ladder;
-    for (int hi = 0; hi < n_heads; ++hi) {
-        const int hh = head0 + hi;
-        const float *src_base = is_q ? sq.q : sq.k;
-        const long long head_off = is_q ? hh * sq.q_head_stride : hh * sq.kv_head_stride;
-        const long long tok_stride = is_q ? sq.q_tok_stride : sq.kv_tok_stride;
-        for (int t0 = tid >> 6; t0 < n_tok; t0 += 4 * kBatch) {
-            float x0[kBatch], x1[kBatch];
-            float2 cs[kBatch];
+    float4 x[kRows];
 #pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                const int t = t0 + 4 * u;
-                x0[u] = x1[u] = 0.f;
-                cs[u] = make_float2(1.f, 0.f);
-                if (t < n_tok) {
-                    const long long src = head_off + (t_begin + t) * tok_stride;
-                    x0[u] = ld_act(src_base, src + i0, in_f16);
-                    x1[u] = ld_act(src_base, src + i1, in_f16);
-                    if (rotated) {
-                        // derived ids (chatglm.cpp:1142-1153, 1319-1327 with n_past = 0), as selects: a branch here
-                        // would split the batch of loads into one round trip per token
-                        const int s_tok = t_begin + t;
-                        const int by_pos = v1 ? (cs_stream ? max(s_tok - v1_lim, 0) : min(s_tok, v1_lim)) : s_tok;
-                        const int row = table_by_position ? by_pos : t;
-                        cs[u] = __ldg(tab + row * 32);
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kBatch; ++u) {
-                const int t = t0 + 4 * u;
-                if (t >= n_tok) continue;
-                const int s = t_begin + t;
-                float y0 = x0[u], y1 = x1[u];
-                if (rotated) rope_rotate(x0[u], x1[u], cs[u].x, cs[u].y, y0, y1);
-                if (is_q) {
-                    __half *dst = q_half + (static_cast<long long>(hh) * s_pad + s) * kD;
-                    if (i1 == i0 + 1) {   // adjacent pair: one 4-byte store
-                        *reinterpret_cast<__half2 *>(dst + i0) =
-                            __halves2half2(__float2half_rn(__fmul_rn(y0, sh.scale)), __float2half_rn(__fmul_rn(y1, sh.scale)));
-                    } else {
-                        dst[i0] = __float2half_rn(__fmul_rn(y0, sh.scale));
-                        dst[i1] = __float2half_rn(__fmul_rn(y1, sh.scale));
-                    }
-                    if (sq.q_roped) {
-                        float *qr = sq.q_roped + (static_cast<long long>(s) * H + hh) * kD;
-                        qr[i0] = y0; qr[i1] = y1;
-                    }
+    for (int u = 0; u < kRows; ++u) {
+        const int t = warp * kRows + u;
+        const long long e = (t_begin + t) * sq.kv_tok_stride + g * sq.kv_head_stride + 4 * lane;
+        x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n_tok) {
+            if (in_f16) {
+                if (vec) {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const __half *>(sq.v) + e));
+                    x[u].x = __uint_as_float(v.x);   // widened behind the loop: nothing here waits for a load
+                    x[u].y = __uint_as_float(v.y);
                 } else {
-                    uint16_t *krow = k_base + (static_cast<long long>(sq.slot * G + hh) * M + sq.kv_before + s) * kD;
-                    if (i1 == i0 + 1) {
-                        *reinterpret_cast<__half2 *>(krow + i0) = __halves2half2(__float2half_rn(y0), __float2half_rn(y1));
-                    } else {
-                        krow[i0] = __half_as_ushort(__float2half_rn(y0));
-                        krow[i1] = __half_as_ushort(__float2half_rn(y1));
-                    }
-                    if (sq.k_roped) {
-                        float *kr = sq.k_roped + (static_cast<long long>(s) * G + hh) * kD;
-                        kr[i0] = y0; kr[i1] = y1;
-                    }
+                    const unsigned short *p = reinterpret_cast<const unsigned short *>(sq.v) + e;
+                    x[u].x = __uint_as_float(p[0] | p[1] << 16);
+                    x[u].y = __uint_as_float(p[2] | p[3] << 16);
                 }
+            } else if (vec) {
+                x[u] = __ldg(reinterpret_cast<const float4 *>(sq.v + e));
+            } else {
+                x[u] = make_float4(__ldg(sq.v + e), __ldg(sq.v + e + 1), __ldg(sq.v + e + 2), __ldg(sq.v + e + 3));
+            }
+        }
+    }
+    if (in_f16) {
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) {
+            const uint32_t w0 = __float_as_uint(x[u].x), w1 = __float_as_uint(x[u].y);
+            const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&w0)), c = __half22float2(*reinterpret_cast<const __half2 *>(&w1));
+            x[u] = make_float4(a.x, a.y, c.x, c.y);
+        }
+    }
+    static_assert(kRows == 8, "a warp's token rows are one 16-byte chunk of every dim");
+    const int place = warp ^ (lane & 7);
+    tile[4 * lane][place] = make_uint4(pack_half2(x[0].x, x[1].x), pack_half2(x[2].x, x[3].x), pack_half2(x[4].x, x[5].x), pack_half2(x[6].x, x[7].x));
+    tile[4 * lane + 1][place] = make_uint4(pack_half2(x[0].y, x[1].y), pack_half2(x[2].y, x[3].y), pack_half2(x[4].y, x[5].y), pack_half2(x[6].y, x[7].y));
+    tile[4 * lane + 2][place] = make_uint4(pack_half2(x[0].z, x[1].z), pack_half2(x[2].z, x[3].z), pack_half2(x[4].z, x[5].z), pack_half2(x[6].z, x[7].z));
+    tile[4 * lane + 3][place] = make_uint4(pack_half2(x[0].w, x[1].w), pack_half2(x[2].w, x[3].w), pack_half2(x[4].w, x[5].w), pack_half2(x[6].w, x[7].w));
+    __syncthreads();
+    uint16_t *vrow0 = v_base + row * kD * M + sq.kv_before + t_begin;
+    const bool vec_row = ((sq.kv_before + t_begin) & 7) == 0;   // M is a multiple of 8: every row is then 16-byte aligned
+    for (int idx = threadIdx.x; idx < kD * (kAppTokens / 8); idx += kAppThreads) {
+        const int d = idx / (kAppTokens / 8), c = idx % (kAppTokens / 8), t = 8 * c;
+        if (t >= n_tok) continue;
+        const uint4 v = tile[d][c ^ (d >> 2 & 7)];
+        uint16_t *dst = vrow0 + static_cast<long long>(d) * M + t;
+        if (vec_row && t + 8 <= n_tok) {
+            *reinterpret_cast<uint4 *>(dst) = v;
+        } else {
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                if (t + e < n_tok) dst[e] = static_cast<uint16_t>(e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
             }
         }
     }
 }
 
-// ---- launch 2: attention ----------------------------------------------------------------------------------------
-// q_map: f16 {D, s_pad, H}, box 64 x 128.  k_map: f16 {D, L, slots*G}, box 64 x 128.  v_map: f16 {L, slots*G*D},
-// box 64 x 128.  L = n_virtual + S is the attended length of the last row.
-//
-// Buffer hand-offs for KV tile j (b = j & 1; every barrier is used once per two tiles, parity (j >> 1) & 1):
-//   k_full[b]   TMA            -> control   K[b] landed      (K[b] is reloaded as soon as S(j) has completed)
-//   v_full[b]   TMA            -> control   V^T[b] landed    (V^T[b] is reloaded once P V(j) has completed)
-//   s_done[b]   tensor core    -> both      S[b] = Q K^T(j) written; K[b] has been read
-//   p_ready[b]  softmax (x4)   -> control   P[b] written (and S[b] read): P V(j) may be issued, S[b] may be reused
-//   o_done[b]   tensor core    -> both      O += P V(j) done; K/V^T[b] and P[b] have been read
+// ---- launch 2: attention ----------------------------------------------------------------------------------------------------
+// What a CTA works on at a time: two q tiles (one in kPrefillSingle) that read the same kv head.
+struct Unit {
+    int seq;
+    int g;            // kv head
+    int head[2];      // q head of each group's tile
+    int tile[2];      // q row tile of each group's tile
+    int n_step;       // 64-token steps, the same for both groups (a tile that ends earlier sees masked steps)
+    bool store1;      // false: there is no second tile, group 1 repeats the first one and stores nothing
+};
+__device__ __forceinline__ Unit unit_of(const PrefillTable &tab, const AttnShape &sh, int idx) {
+    Unit un;
+    un.seq = 0;
+    while (un.seq + 1 < tab.n_seq && idx >= tab.seqs[un.seq + 1].unit_begin) ++un.seq;
+    const PrefillSeq &ps = tab.seqs[un.seq];
+    const int u = idx - ps.unit_begin, n_q = ps.n_q;
+    un.store1 = true;
+    // the longest row tiles first
+    if (tab.mode == kPrefillSingle) {
+        un.tile[0] = un.tile[1] = n_q - 1 - u / sh.H;
+        un.head[0] = un.head[1] = u % sh.H;
+    } else if (tab.mode == kPrefillPairHeads) {
+        const int per_kv = (sh.R + 1) / 2, hu = u % (sh.G * per_kv);
+        un.tile[0] = un.tile[1] = n_q - 1 - u / (sh.G * per_kv);
+        un.head[0] = hu / per_kv * sh.R + 2 * (hu % per_kv);
+        un.store1 = 2 * (hu % per_kv) + 1 < sh.R;
+        un.head[1] = un.head[0] + (un.store1 ? 1 : 0);
+    } else {
+        const int p = (n_q + 1) / 2 - 1 - u / sh.H;
+        un.tile[0] = 2 * p;
+        un.store1 = 2 * p + 1 < n_q;
+        un.tile[1] = un.tile[0] + (un.store1 ? 1 : 0);
+        un.head[0] = un.head[1] = u % sh.H;
+    }
+    un.g = un.head[0] / sh.R;
+    const int L = ps.sq.kv_before + ps.sq.qlen;
+    const int end = ps.causal ? min(L, ps.sq.kv_before + (un.tile[1] + 1) * kQTile) : L;   // one past the last visible token
+    un.n_step = (end + kStep - 1) / kStep;
+    return un;
+}
+// The units are dealt to the CTAs in rows of gridDim.x, every other row backwards: the k-th unit of this CTA (past the end: none
+// left).  Units come longest first, so the shares come out even.
+__device__ __forceinline__ int unit_index(int k) {
+    const int n = gridDim.x, b = blockIdx.x;
+    return k * n + ((k & 1) ? n - 1 - b : b);
+}
+
+// q row pairs p0, p0 + step, ... of the unit's tiles (64 pairs per tile) by one warp: load, rotate, scale, round to f16 and
+// store at the places of the swizzled A operand.  at(w): where tile w goes, shared memory or the global image of it; kRows row
+// pairs have their loads in flight together.
+template <int kPairs, class At>
+__device__ __forceinline__ void stage_q(const PrefillSeq &ps, const AttnShape &sh, const Unit &un, int n_groups, int p0, int step, int lane, At at) {
+    const SeqDev &sq = ps.sq;
+    const int hl = lane & 15, sub = lane >> 4;
+    const bool f16 = (sq.flags & CGLM_SEQ_QKV_F16) != 0;
+#pragma unroll 1
+    for (int p = p0; p < 64 * n_groups; p += kPairs * step) {
+        Row8 x[kPairs];
+#pragma unroll
+        for (int u = 0; u < kPairs; ++u) {
+            const int pu = min(p + u * step, 64 * n_groups - 1), w = pu >> 6, r = 2 * (pu & 63) + sub;   // past the end: the last pair again
+            load_row8(x[u], ps, sh.rope_type, sq.q, (w ? un.head[1] : un.head[0]) * sq.q_head_stride, sq.q_tok_stride,
+                      (w ? un.tile[1] : un.tile[0]) * kQTile + r, hl);
+        }
+#pragma unroll
+        for (int u = 0; u < kPairs; ++u) {
+            const int pu = min(p + u * step, 64 * n_groups - 1), w = pu >> 6, r = 2 * (pu & 63) + sub;
+            float y[8];
+            rotate_row8(x[u], f16, sh.rope_type, hl, y);
+            const int s = (w ? un.tile[1] : un.tile[0]) * kQTile + r;
+            if (sq.q_roped && s < sq.qlen) st_f32x8(sq.q_roped + (static_cast<long long>(s) * sh.H + (w ? un.head[1] : un.head[0])) * kD + 8 * hl, y);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = __fmul_rn(y[i], sh.scale);
+            *reinterpret_cast<uint4 *>(at(w) + (hl >> 3) * kHalfBytes + r * 128 + (((hl & 7) ^ (r & 7)) << 4)) = pack_half8(y);
+        }
+    }
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
+                 "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+// 32 bytes of one thread to global memory: one full sector per lane
+__device__ __forceinline__ void st_sector(void *p, const uint32_t (&v)[8], int align) {
+    if (align >= 32) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                     "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+    } else if (align >= 16) {
+        reinterpret_cast<uint4 *>(p)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<uint4 *>(p)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) reinterpret_cast<uint2 *>(p)[i] = make_uint2(v[2 * i], v[2 * i + 1]);
+    }
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
-prefill_attn_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
-                    const __grid_constant__ CUtensorMap v_map, AttnShape sh, int S, int kv_row0, float *__restrict__ out,
-                    int out_f16, WsHeader *hdr) {
+prefill_attn_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ PrefillTable tab, AttnShape sh, int n_units,
+                    uint8_t *__restrict__ q_scratch, WsHeader *hdr) {
     extern __shared__ uint8_t smem_raw[];
     PrefillSmem &sm = *reinterpret_cast<PrefillSmem *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // A CTA takes q tile (n_q - 1 - x) and then q tile x of one head: under the causal mask the first sees the most
-    // KV tiles and the second the fewest, so every CTA of the grid has the same amount of work.
-    const int h = blockIdx.y;
-    const int n_q = (S + kQTile - 1) / kQTile;
-    const int V = sh.V, L = V + S;
-    const int kv_row = kv_row0 + h / sh.R;
-    const bool causal = sh.mask_type == CGLM_MASK_CAUSAL;
-    const int q_tiles[2] = {n_q - 1 - static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.x)};
-    const int n_pass = q_tiles[0] == q_tiles[1] ? 1 : 2;
-    auto kv_tiles_of = [&](int q_tile) {
-        const int last_visible = causal ? min(L, V + q_tile * kQTile + kQTile) : L;   // one past the last visible token
-        return (last_visible + kKvTile - 1) / kKvTile;
-    };
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // the same in every lane, and known to be
+    const int n_groups = tab.mode == kPrefillSingle ? 1 : 2;
 
     if (tid == 0) {
         sm.abort_flag = 0;
-        mbar_init(&sm.q_full, 1);
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&sm.k_full[b], 1);
-            mbar_init(&sm.v_full[b], 1);
-            mbar_init(&sm.s_done[b], 1);
-            mbar_init(&sm.p_ready[b], kSoftmaxThreads / 32);
-            mbar_init(&sm.o_done[b], 1);
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(&sm.kv_full[s], 1);
+            mbar_init(&sm.kv_empty[s], n_groups);
+        }
+        for (int w = 0; w < 2; ++w) {
+            mbar_init(&sm.q_full[w], 1);
+            mbar_init(&sm.q_empty[w], 1);
+            mbar_init(&sm.s_full[w], 1);
+            mbar_init(&sm.s_empty[w], kGroupThreads / 32);
+            mbar_init(&sm.p_full[w][0], kGroupThreads / 32);   // two: a group may be a step ahead of its MMA warp
+            mbar_init(&sm.p_full[w][1], kGroupThreads / 32);
+            mbar_init(&sm.o_step[w], 1);
+            mbar_init(&sm.o_full[w], 1);
+            mbar_init(&sm.o_empty[w], kGroupThreads / 32);
         }
         fence_mbar_init();
     }
-    if (warp == 0) {
+    if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
                      "r"(kTmemCols)
                      : "memory");
@@ -320,269 +492,303 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = sm.tmem_base;
-    // Launched as a programmatic dependent of the prepare kernel: everything above overlapped its tail; its q, K and
-    // V^T are read from here on.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
 
-    // j: running tile count of the CTA (buffer j & 1, barrier parity (j >> 1) & 1); jl: KV tile index inside a pass.
-    // Loads, score MMAs and P V MMAs are issued by three different warps, each a plain loop over the tiles that
-    // waits only for what its own step needs: the next score tile is computed while the softmax warps work on the
-    // current one, P V(j) follows as soon as they are done, and no step queues behind another step's barrier.
-    if (warp == kLoadWarp) {
-        // ================================ load warp: TMA ===================================================
-        if (lane == 0) {
-            tma_prefetch_desc(&q_map);
-            tma_prefetch_desc(&k_map);
-            tma_prefetch_desc(&v_map);
-        }
-        int jt0 = 0;
-        for (int pass = 0; pass < n_pass; ++pass) {
-            const int s0 = q_tiles[pass] * kQTile;
-            const int n_kv = kv_tiles_of(q_tiles[pass]);
-            if (lane == 0) {
-                mbar_arrive_expect_tx(&sm.q_full, kTileBytes);
-                tma_load_3d(sm.q, &q_map, 0, s0, h, &sm.q_full);
-                tma_load_3d(sm.q + kHalfBytes, &q_map, 64, s0, h, &sm.q_full);
-                for (int jl = 0; jl < n_kv; ++jl) {
-                    const int j = jt0 + jl, b = j & 1;
-                    // K[b] was read by S(j-2), V^T[b] by P V(j-2); at the start of a pass both buffers are free
-                    if (jl >= 2) mbar_wait_bounded(&sm.s_done[b], ((j - 2) >> 1) & 1u, &sm.abort_flag);
-                    mbar_arrive_expect_tx(&sm.k_full[b], kTileBytes);
-                    tma_load_3d(sm.k[b], &k_map, 0, jl * kKvTile, kv_row, &sm.k_full[b]);
-                    tma_load_3d(sm.k[b] + kHalfBytes, &k_map, 64, jl * kKvTile, kv_row, &sm.k_full[b]);
-                    if (jl >= 2) mbar_wait_bounded(&sm.o_done[b], ((j - 2) >> 1) & 1u, &sm.abort_flag);
-                    mbar_arrive_expect_tx(&sm.v_full[b], kTileBytes);
-                    tma_load_2d(sm.v[b], &v_map, jl * kKvTile, kv_row * kD, &sm.v_full[b]);
-                    tma_load_2d(sm.v[b] + kHalfBytes, &v_map, jl * kKvTile + 64, kv_row * kD, &sm.v_full[b]);
+    if (warp < kLoadWarp) {
+        // The first unit's q rows straight into shared memory, by every warp that has nothing else to do yet.  They are the call's
+        // input: final once the append kernel has started, which this grid's launch implies.
+        const Unit un = unit_of(tab, sh, unit_index(0));   // the grid has no more CTAs than there are units
+        stage_q<4>(tab.seqs[un.seq], sh, un, n_groups, warp, kLoadWarp, lane, [&](int w) { return sm.q[w]; });
+        fence_proxy_async();   // plain stores above, the tensor core reads through the async proxy
+        named_bar_sync(4, 32 * kLoadWarp);
+        if (tid < n_groups) mbar_arrive(&sm.q_full[tid]);
+        __syncwarp();
+    }
+    if (warp >= kQWarp) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+        if (warp < kLoadWarp) {
+            // ================================ q warps: tiles of the CTA's second and later units ===========================
+            // The tile is staged in global memory (L2), already in the order of the swizzled operand, while the previous unit
+            // runs, and copied in when that unit's last scores have been computed: a unit starts without a round trip for q.
+            const int qw = warp - kQWarp;
+            uint8_t *scratch = q_scratch + static_cast<size_t>(blockIdx.x) * 2 * kTileBytes;
+            for (int k = 1, idx; (idx = unit_index(k)) < n_units; ++k) {
+                const Unit un = unit_of(tab, sh, idx);
+                const PrefillSeq &ps = tab.seqs[un.seq];
+                if (k > 1) {   // the previous tiles have left the scratch
+                    for (int w = 0; w < n_groups; ++w) mbar_wait_bounded(&sm.q_full[w], (k - 1) & 1, &sm.abort_flag);
                 }
-            }
-            jt0 += n_kv;
-            __syncwarp();
-            if (pass + 1 < n_pass) {
-                // the next pass reloads Q, K, V^T: every MMA of this pass must have read them, and the softmax
-                // warps must be done with the output staging tile that overlays the K/V^T buffers
-                named_bar_sync(2, kThreads);
-            }
-        }
-    } else if (warp == kScoreWarp) {
-        // ================================ score warp: one thread issues S(j) = Q K(j)^T ======================
-        int jt0 = 0;
-        for (int pass = 0; pass < n_pass; ++pass) {
-            const int n_kv = kv_tiles_of(q_tiles[pass]);
-            if (lane == 0) {
-                mbar_wait_bounded(&sm.q_full, pass & 1u, &sm.abort_flag);
-                for (int jl = 0; jl < n_kv; ++jl) {
-                    const int j = jt0 + jl, b = j & 1;
-                    mbar_wait_bounded(&sm.k_full[b], (j >> 1) & 1u, &sm.abort_flag);
-                    // S[b] was last read by the softmax of tile j-2
-                    if (jl >= 2) mbar_wait_bounded(&sm.p_ready[b], ((j - 2) >> 1) & 1u, &sm.abort_flag);
-                    tc_fence_after();
-#pragma unroll
-                    for (int kh = 0; kh < 2; ++kh) {
-#pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            umma_f16(tmem + 128 * b, smem_desc(smem_u32(sm.q) + kh * kHalfBytes + ks * 32),
-                                     smem_desc(smem_u32(sm.k[b]) + kh * kHalfBytes + ks * 32), (kh | ks) != 0);
-                        }
+                __syncwarp();
+                stage_q<2>(ps, sh, un, n_groups, qw, 4, lane, [&](int w) { return scratch + w * kTileBytes; });
+                __threadfence();
+                asm volatile("fence.proxy.async;" ::: "memory");   // plain stores above, the bulk copy reads through the async proxy
+                named_bar_sync(3, 128);
+                if (warp == kQWarp && lane == 0) {
+                    asm volatile("fence.proxy.async;" ::: "memory");
+                    for (int w = 0; w < n_groups; ++w) {
+                        mbar_wait_bounded(&sm.q_empty[w], (k - 1) & 1, &sm.abort_flag);
+                        mbar_arrive_expect_tx(&sm.q_full[w], kTileBytes);
+                        bulk_load(sm.q[w], scratch + w * kTileBytes, kTileBytes, &sm.q_full[w]);
                     }
-                    umma_commit(&sm.s_done[b]);
                 }
+                __syncwarp();
             }
-            jt0 += n_kv;
-            __syncwarp();
-            if (pass + 1 < n_pass) {
-                named_bar_sync(2, kThreads);
-            }
-        }
-    } else if (warp == kPvWarp) {
-        // ================================ PV warp: one thread issues O (+)= P(j) V(j) =========================
-        int jt0 = 0;
-        for (int pass = 0; pass < n_pass; ++pass) {
-            const int n_kv = kv_tiles_of(q_tiles[pass]);
+        } else if (warp == kLoadWarp) {
+            // ================================ load warp: K(0), V(0), K(1), V(1), ... through the ring =====================
             if (lane == 0) {
-                for (int jl = 0; jl < n_kv; ++jl) {
-                    const int j = jt0 + jl, b = j & 1;
-                    // any rescale of O for the tile precedes p_ready
-                    mbar_wait_bounded(&sm.v_full[b], (j >> 1) & 1u, &sm.abort_flag);
-                    mbar_wait_bounded(&sm.p_ready[b], (j >> 1) & 1u, &sm.abort_flag);
-                    tc_fence_after();
-#pragma unroll
-                    for (int th = 0; th < 2; ++th) {
-#pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            umma_f16(tmem + 256, smem_desc(smem_u32(sm.p[b]) + th * kHalfBytes + ks * 32),
-                                     smem_desc(smem_u32(sm.v[b]) + th * kHalfBytes + ks * 32), (jl | th | ks) != 0);
+                tma_prefetch_desc(&k_map);
+                asm volatile("griddepcontrol.wait;" ::: "memory");   // the append kernel's K rows and V^T columns are in place
+                int st = 0;
+                uint32_t parity = 1;   // a fresh barrier counts as the completed phase before its first one
+                for (int k = 0, idx; (idx = unit_index(k)) < n_units; ++k) {
+                    const Unit un = unit_of(tab, sh, idx);
+                    const CUtensorMap *v_map = &tab.v_map[un.seq];
+                    const int kv_row = tab.seqs[un.seq].sq.slot * sh.G + un.g, n_tiles = (un.n_step + 1) / 2;
+                    for (int i = 0; i < 2 * n_tiles; ++i) {
+                        const int j = i >> 1;
+                        mbar_wait_bounded(&sm.kv_empty[st], parity, &sm.abort_flag);
+                        mbar_arrive_expect_tx(&sm.kv_full[st], kTileBytes);
+                        if ((i & 1) == 0) {
+                            tma_load_3d(sm.kv[st], &k_map, 0, j * kKvTile, kv_row, &sm.kv_full[st]);
+                            tma_load_3d(sm.kv[st] + kHalfBytes, &k_map, 64, j * kKvTile, kv_row, &sm.kv_full[st]);
+                        } else {
+                            tma_load_2d(sm.kv[st], v_map, j * kKvTile, kv_row * kD, &sm.kv_full[st]);
+                            tma_load_2d(sm.kv[st] + kHalfBytes, v_map, j * kKvTile + 64, kv_row * kD, &sm.kv_full[st]);
                         }
+                        if (++st == kStages) { st = 0; parity ^= 1; }
                     }
-                    umma_commit(&sm.o_done[b]);
                 }
+                // every load of this CTA is on its way: the next kernel of the stream may take the places that free up
+                asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             }
-            jt0 += n_kv;
-            __syncwarp();
-            if (pass + 1 < n_pass) {
-                named_bar_sync(2, kThreads);
+        } else if (warp < kMmaWarp + n_groups) {
+            // ================================ MMA warp of group w ========================================================
+            // One warp per group: a wait of one leaves the tensor pipe to the other (one warp for both spent half of
+            // its time between two MMAs).
+            const int w = warp - kMmaWarp;
+            const uint32_t kv_desc0 = desc_lo(smem_u32(sm.kv[0])), q_desc = desc_lo(smem_u32(sm.q[w]));
+            const uint32_t t_s = tmem + 128 * w, t_o = tmem + 256 + 128 * w, lead = elect_one();
+            // A place in the CTA's sequence of steps: step s (of n) of its k-th unit, the ring stage of its tile.  The scores
+            // run one step ahead of the P V.
+            struct Cursor {
+                int k, s, n, st;
+                uint32_t parity;
+            };
+            auto open = [&](Cursor &c) {   // first step of unit c.k, if there is one
+                const int idx = unit_index(c.k);
+                c.s = 0;
+                c.n = idx < n_units ? unit_of(tab, sh, idx).n_step : 0;
+            };
+            auto advance = [&](Cursor &c) {
+                ++c.s;
+                if ((c.s & 1) == 0 || c.s == c.n) {   // K and V^T tiles alternate in the ring
+                    c.st += 2;
+                    if (c.st >= kStages) { c.st -= kStages; c.parity ^= 1; }
+                }
+                if (c.s == c.n) { ++c.k; open(c); }
+            };
+            Cursor cs{0, 0, 0, 0, 0}, cp{0, 0, 0, 1, 0};
+            open(cs);
+            open(cp);
+            auto scores = [&](int t) {   // Q K^T of step cs, the CTA's t-th
+                const int half = cs.s & 1;
+                if (half == 0) mbar_wait_bounded(&sm.kv_full[cs.st], cs.parity, &sm.abort_flag);
+                if (cs.s == 0) mbar_wait_bounded(&sm.q_full[w], cs.k & 1, &sm.abort_flag);
+                if (t > 0) mbar_wait_bounded(&sm.s_empty[w], (t - 1) & 1, &sm.abort_flag);
+                const uint32_t b = kv_desc0 + ((cs.st * kTileBytes + half * kStep * 128) >> 4);
+                const bool last = cs.s + 1 == cs.n;
+                __syncwarp();
+                tc_fence_after();
+                umma_ss<kIdescS, false>(t_s, q_desc, b, lead);
+#pragma unroll
+                for (int ks = 1; ks < 8; ++ks) {
+                    const int off = ((ks >> 2) * kHalfBytes + (ks & 3) * 32) >> 4;
+                    umma_ss<kIdescS, true>(t_s, q_desc + off, b + off, lead);
+                }
+                umma_commit(&sm.s_full[w], lead);
+                if (half == 1 || last) umma_commit(&sm.kv_empty[cs.st], lead);
+                if (last) umma_commit(&sm.q_empty[w], lead);
+                advance(cs);
+            };
+            if (cs.n > 0) scores(0);
+            for (int t = 0; cp.n > 0; ++t) {
+                // the next scores as soon as the softmax has those of step t in registers; at the end of a unit, whose successor's q
+                // tile may not be there yet, behind the P V
+                const bool ahead = cs.n > 0 && cs.s > 0;
+                if (ahead) scores(t + 1);
+                const int half = cp.s & 1;
+                if (half == 0) mbar_wait_bounded(&sm.kv_full[cp.st], cp.parity, &sm.abort_flag);
+                if (cp.s == 0 && cp.k > 0) mbar_wait_bounded(&sm.o_empty[w], (cp.k - 1) & 1, &sm.abort_flag);
+                mbar_wait_bounded(&sm.p_full[w][t & 1], (t >> 1) & 1, &sm.abort_flag);   // P(t) written, any rescale of O done
+                const uint32_t b = kv_desc0 + ((cp.st * kTileBytes + half * kHalfBytes) >> 4);
+                const uint32_t a = t_s + 64 + 32 * (t & 1);
+                const bool last = cp.s + 1 == cp.n;
+                __syncwarp();
+                tc_fence_after();
+                umma_ts<kIdescO>(t_o, a, b, cp.s != 0, lead);
+#pragma unroll
+                for (int ks = 1; ks < kStep / 16; ++ks) umma_ts<kIdescO>(t_o, a + 8 * ks, b + (ks * 32 >> 4), 1, lead);
+                umma_commit(&sm.o_step[w], lead);
+                if (half == 1 || last) umma_commit(&sm.kv_empty[cp.st], lead);
+                if (last) umma_commit(&sm.o_full[w], lead);
+                advance(cp);
+                if (!ahead && cs.n > 0) scores(t + 1);
             }
         }
     } else {
-        // ================================ softmax warps: one q row per thread =================================
-        const uint32_t lane_base = static_cast<uint32_t>(32 * warp) << 16;   // this warp's quarter of the TMEM lanes
-        const uint32_t to = tmem + 256 + lane_base;
-        int jt0 = 0;
-      for (int pass = 0; pass < n_pass; ++pass) {
-        const int s0 = q_tiles[pass] * kQTile;
-        const int n_kv = kv_tiles_of(q_tiles[pass]);
-        const int s_row = s0 + tid;             // this thread's q row (may lie past S in the last q tile)
-        float m_ref = -INFINITY, l_run = 0.f;   // reference maximum (log2 domain) and row sum relative to it
-        // the last token a row may attend (inclusive)
-        const int row_last = causal ? min(L - 1, V + s_row) : (s_row < S - 1 ? L - 2 : L - 1);
-
-        for (int jl = 0; jl < n_kv; ++jl) {
-            const int j = jt0 + jl;
-            const int b = j & 1;
-            mbar_wait_bounded(&sm.s_done[b], (j >> 1) & 1u, &sm.abort_flag);
-            tc_fence_after();
-            const uint32_t ts = tmem + 128 * b + lane_base;
-            const int t0 = jl * kKvTile;
-            // the whole score row of this tile: 4 loads in flight, one wait
-            float sv[kKvTile];
-            {
-                uint32_t *r = reinterpret_cast<uint32_t *>(sv);
-#pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                        "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                        : "=r"(r[32 * ch + 0]), "=r"(r[32 * ch + 1]), "=r"(r[32 * ch + 2]), "=r"(r[32 * ch + 3]),
-                          "=r"(r[32 * ch + 4]), "=r"(r[32 * ch + 5]), "=r"(r[32 * ch + 6]), "=r"(r[32 * ch + 7]),
-                          "=r"(r[32 * ch + 8]), "=r"(r[32 * ch + 9]), "=r"(r[32 * ch + 10]), "=r"(r[32 * ch + 11]),
-                          "=r"(r[32 * ch + 12]), "=r"(r[32 * ch + 13]), "=r"(r[32 * ch + 14]), "=r"(r[32 * ch + 15]),
-                          "=r"(r[32 * ch + 16]), "=r"(r[32 * ch + 17]), "=r"(r[32 * ch + 18]), "=r"(r[32 * ch + 19]),
-                          "=r"(r[32 * ch + 20]), "=r"(r[32 * ch + 21]), "=r"(r[32 * ch + 22]), "=r"(r[32 * ch + 23]),
-                          "=r"(r[32 * ch + 24]), "=r"(r[32 * ch + 25]), "=r"(r[32 * ch + 26]), "=r"(r[32 * ch + 27]),
-                          "=r"(r[32 * ch + 28]), "=r"(r[32 * ch + 29]), "=r"(r[32 * ch + 30]), "=r"(r[32 * ch + 31])
-                        : "r"(ts + ch * 32)
-                        : "memory");
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            }
-            // raw scores stay in sv; the log2(e) factor is folded into the exponent's FMA below.  Four independent
-            // chains each for the maximum and the sum: a 128-long dependent chain would cost more than the math.
-            if (t0 + kKvTile - 1 > row_last) {   // the diagonal tile (or the v1 mask's last column): blank hidden tokens
-#pragma unroll
-                for (int i = 0; i < kKvTile; ++i) {
-                    sv[i] = t0 + i <= row_last ? sv[i] : -INFINITY;
-                }
-            }
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int i = 0; i < kKvTile; i += 8) {
-                mx4[0] = max3(mx4[0], sv[i], sv[i + 1]); mx4[1] = max3(mx4[1], sv[i + 2], sv[i + 3]);
-                mx4[2] = max3(mx4[2], sv[i + 4], sv[i + 5]); mx4[3] = max3(mx4[3], sv[i + 6], sv[i + 7]);
-            }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * kLog2e;
-            // keep the old reference unless the maximum outgrew it by more than the threshold
-            const bool grow = mx > m_ref + kRescaleThreshold;   // also true for the first visible tile (m_ref = -inf)
-            const float m_new = grow ? mx : m_ref;
-            const float alpha = grow ? ex2_approx(m_ref - m_new) : 1.f;   // 0 when m_ref was -inf
-            if (jl > 0 && __any_sync(0xffffffffu, grow)) {
-                // rescale this warp's rows of O in tensor memory; P V(j-1) must have landed first
-                mbar_wait_bounded(&sm.o_done[(j - 1) & 1], ((j - 1) >> 1) & 1u, &sm.abort_flag);
+        // ================================ softmax groups: one q row per thread ========================================
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+        const int w = warp >> 2, gw = warp & 3;   // group, warp inside it
+        const int row = 32 * gw + lane;           // TMEM lane
+        const uint32_t lane_base = static_cast<uint32_t>(32 * gw) << 16;   // this warp's quarter of the TMEM lanes
+        const uint32_t ts = tmem + 128 * w + lane_base, to = tmem + 256 + 128 * w + lane_base;
+        int t = 0;   // steps so far
+        for (int k = 0, idx; w < n_groups && (idx = unit_index(k)) < n_units; ++k) {
+            const Unit un = unit_of(tab, sh, idx);
+            const PrefillSeq &ps = tab.seqs[un.seq];
+            const SeqDev &sq = ps.sq;
+            const int S = sq.qlen, h = w ? un.head[1] : un.head[0], s0 = (w ? un.tile[1] : un.tile[0]) * kQTile, n_step = un.n_step;
+            float m_ref = -INFINITY, l_run = 0.f;   // reference maximum (log2 domain) and row sum relative to it
+            // the last token a row may attend (inclusive); a row past S is computed like any other and not stored
+            const int L = sq.kv_before + S, s_row = s0 + row;
+            const int row_last = ps.causal ? min(L - 1, sq.kv_before + s_row) : (ps.blocked && s_row < S - 1 ? L - 2 : L - 1);
+            // One step: 64 tokens.  Masked and unmasked steps are separate code: in one loop the mask's selects are issued, if
+            // predicated off, in every step.
+            auto step = [&](int j, auto masked) {
+                mbar_wait_bounded(&sm.s_full[w], t & 1, &sm.abort_flag);
+                __syncwarp();   // aligned tensor-memory instructions follow
                 tc_fence_after();
+                float2 sv[kStep / 2];
+                tmem_ld32_nowait(ts, reinterpret_cast<uint32_t *>(sv));
+                tmem_ld32_nowait(ts + 32, reinterpret_cast<uint32_t *>(sv) + 32);
+                tmem_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.s_empty[w]);   // the scores of the next step may follow
+                // raw scores stay in sv; the log2(e) factor is folded into the exponent's FMA below.  Independent chains for
+                // the maximum and the sum: one long dependent chain would cost more than the math.
+                if constexpr (decltype(masked)::value) {
+                    const int last = row_last - j * kStep;
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
-                    float ov[32];
-                    tmem_ld32(to + ch * 32, ov);
-                    asm volatile(
-                        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                        "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-                        ::"r"(to + ch * 32), "f"(ov[0] * alpha), "f"(ov[1] * alpha), "f"(ov[2] * alpha), "f"(ov[3] * alpha),
-                          "f"(ov[4] * alpha), "f"(ov[5] * alpha), "f"(ov[6] * alpha), "f"(ov[7] * alpha), "f"(ov[8] * alpha),
-                          "f"(ov[9] * alpha), "f"(ov[10] * alpha), "f"(ov[11] * alpha), "f"(ov[12] * alpha),
-                          "f"(ov[13] * alpha), "f"(ov[14] * alpha), "f"(ov[15] * alpha), "f"(ov[16] * alpha),
-                          "f"(ov[17] * alpha), "f"(ov[18] * alpha), "f"(ov[19] * alpha), "f"(ov[20] * alpha),
-                          "f"(ov[21] * alpha), "f"(ov[22] * alpha), "f"(ov[23] * alpha), "f"(ov[24] * alpha),
-                          "f"(ov[25] * alpha), "f"(ov[26] * alpha), "f"(ov[27] * alpha), "f"(ov[28] * alpha),
-                          "f"(ov[29] * alpha), "f"(ov[30] * alpha), "f"(ov[31] * alpha)
-                        : "memory");
+                    for (int i = 0; i < kStep / 2; ++i) {
+                        sv[i].x = 2 * i <= last ? sv[i].x : -INFINITY;
+                        sv[i].y = 2 * i + 1 <= last ? sv[i].y : -INFINITY;
+                    }
                 }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            }
-            const float m_base = m_new == -INFINITY ? 0.f : m_new;   // a row that has seen nothing yet: every p is 0
-            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-            // P[b] was last read by P V(j-2), issued by another thread than S(j): wait for it explicitly
-            if (jl >= 2) mbar_wait_bounded(&sm.o_done[b], ((j - 2) >> 1) & 1u, &sm.abort_flag);
+                float mx4[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(sv[c].x, sv[c].y);
+#pragma unroll
+                for (int i = 4; i < kStep / 2; ++i) mx4[i & 3] = max3(mx4[i & 3], sv[i].x, sv[i].y);
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * kLog2e;
+                // keep the old reference unless the maximum outgrew it by more than the threshold
+                const bool grow = mx > m_ref + kRescaleThreshold;   // also true for the first visible step (m_ref = -inf)
+                if (__any_sync(0xffffffffu, grow)) {
+                    const float m_new = grow ? mx : m_ref;
+                    const float alpha = grow ? ex2_approx(m_ref - m_new) : 1.f;   // 0 when m_ref was -inf
+                    l_run *= alpha;
+                    m_ref = m_new;
+                    if (j > 0) {
+                        // rescale this warp's rows of O: P V(t - 1) must have landed (P V(t - 2) has: it precedes the scores of t)
+                        mbar_wait_bounded(&sm.o_step[w], (t - 1) & 1, &sm.abort_flag);
+                        __syncwarp();
+                        tc_fence_after();
+#pragma unroll 1
+                        for (int ch = 0; ch < 8; ++ch) {
+                            uint32_t ov[16];
+                            asm volatile(
+                                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+                                "tcgen05.wait::ld.sync.aligned;"
+                                : "=r"(ov[0]), "=r"(ov[1]), "=r"(ov[2]), "=r"(ov[3]), "=r"(ov[4]), "=r"(ov[5]), "=r"(ov[6]), "=r"(ov[7]),
+                                  "=r"(ov[8]), "=r"(ov[9]), "=r"(ov[10]), "=r"(ov[11]), "=r"(ov[12]), "=r"(ov[13]), "=r"(ov[14]), "=r"(ov[15])
+                                : "r"(to + ch * 16)
+                                : "memory");
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+                            tmem_st16(to + ch * 16, ov);
+                        }
+                    }
+                }
+                const float m_base = decltype(masked)::value && m_ref == -INFINITY ? 0.f : m_ref;   // a row that has seen nothing yet: every p is 0
+                const float2 lg = make_float2(kLog2e, kLog2e), mb = make_float2(-m_base, -m_base);
+                float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                for (int ch = 0; ch < kStep / 32; ++ch) {
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        float2 e = __ffma2_rn(sv[16 * ch + i], lg, mb);   // masked scores are -inf: p = 0
+                        e.x = ex2_approx(e.x);
+                        e.y = ex2_approx(e.y);
+                        sum[i & 1] = __fadd2_rn(sum[i & 1], e);
+                        packed[i] = pack_half2(e.x, e.y);
+                    }
+                    // tokens [32 ch, 32 ch + 32) of the row: columns [16 ch, 16 ch + 16) of P.  The P V that read this buffer two
+                    // steps ago precedes the scores of this step in the tensor pipe.
+                    tmem_st16(ts + 64 + 32 * (t & 1) + ch * 16, packed);
+                }
+                l_run += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.p_full[w][t & 1]);
+                ++t;
+            };
+            // steps in which every row of this warp sees all 64 tokens
+            const int first_last = ps.causal ? min(L - 1, sq.kv_before + s0 + 32 * gw) : (ps.blocked ? L - 2 : L - 1);
+            const int n_clear = min(n_step, (first_last + 1) / kStep);
+            int j = 0;
+#pragma unroll 1
+            for (; j < n_clear; ++j) step(j, std::false_type{});
+#pragma unroll 1
+            for (; j < n_step; ++j) step(j, std::true_type{});
+
+            // ---- output: context_layer[s][h*D + d] (chatglm.cpp:712-717) straight from tensor memory, 32 bytes of its row per
+            //      store and thread: whole sectors, nothing staged, nobody waited for ------------------------------------------
+            mbar_wait_bounded(&sm.o_full[w], k & 1, &sm.abort_flag);
+            __syncwarp();
+            tc_fence_after();
+            const float inv = 1.f / l_run;
+            const bool out_f16 = (sq.flags & CGLM_SEQ_OUT_F16) != 0, store = s_row < S && (w == 0 || un.store1);
+            const long long at = (static_cast<long long>(s_row) * sh.H + h) * kD;
+            const int align = static_cast<int>(reinterpret_cast<uintptr_t>(sq.out) & 31) == 0 ? 32 : ((reinterpret_cast<uintptr_t>(sq.out) & 15) == 0 ? 16 : 8);
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch) {
-                uint32_t packed[16];
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float e0, e1;
-                    fma2(e0, e1, sv[ch * 32 + i], sv[ch * 32 + i + 1], kLog2e, -m_base);   // masked scores are -inf: p = 0
-                    const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
-                    add2(sum4[2 * ((i >> 1) & 1)], sum4[2 * ((i >> 1) & 1) + 1], p0, p1);
-                    packed[i >> 1] = pack_half2(p0, p1);
+                uint32_t r[32];
+                tmem_ld32_nowait(to + ch * 32, r);
+                tmem_wait_ld();
+                if (ch == 3) {   // all of O has been read: the next unit's P V may overwrite it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sm.o_empty[w]);
                 }
-                // tokens [32ch, 32ch+32) of the tile: half = ch / 2, 16-byte chunks (ch % 2) * 4 .. +3 of the 128-byte row
-                const uint32_t rowaddr = smem_u32(sm.p[b]) + (ch >> 1) * kHalfBytes + tid * 128;
+                if (store) {
+                    if (out_f16) {
 #pragma unroll
-                for (int c4 = 0; c4 < 4; ++c4) {
-                    const int chunk = (ch & 1) * 4 + c4;
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rowaddr + ((chunk ^ (tid & 7)) << 4)),
-                                 "r"(packed[4 * c4]), "r"(packed[4 * c4 + 1]), "r"(packed[4 * c4 + 2]),
-                                 "r"(packed[4 * c4 + 3])
-                                 : "memory");
+                        for (int c = 0; c < 2; ++c) {
+                            uint32_t v[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e)
+                                v[e] = pack_half2(__uint_as_float(r[16 * c + 2 * e]) * inv, __uint_as_float(r[16 * c + 2 * e + 1]) * inv);
+                            st_sector(reinterpret_cast<__half *>(sq.out) + at + 32 * ch + 16 * c, v, align);
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            uint32_t v[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) v[e] = __float_as_uint(__uint_as_float(r[8 * c + e]) * inv);
+                            st_sector(sq.out + at + 32 * ch + 8 * c, v, align);
+                        }
+                    }
                 }
-            }
-            l_run = l_run * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-            m_ref = m_new;
-            fence_proxy_async();      // P was written with plain stores, the tensor core reads it through the async proxy
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_ready[b]);
-        }
-        // all of O has been accumulated once the last P V has landed
-        mbar_wait_bounded(&sm.o_done[(jt0 + n_kv - 1) & 1], ((jt0 + n_kv - 1) >> 1) & 1u, &sm.abort_flag);
-        tc_fence_after();
-
-        // ---- output: context_layer[s][h*D + d] (chatglm.cpp:712-717), staged through shared memory so that the
-        //      global stores of a warp cover whole rows.  All MMAs have completed: the K/V^T buffers are free. ------
-        named_bar_sync(1, kSoftmaxThreads);
-        float *stage = reinterpret_cast<float *>(sm.k[0]);
-        const float inv = 1.f / l_run;
-#pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-            float ov[32];
-            tmem_ld32(to + ch * 32, ov);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                *reinterpret_cast<float4 *>(&stage[tid * kOutStride + ch * 32 + 4 * i]) =
-                    make_float4(ov[4 * i] * inv, ov[4 * i + 1] * inv, ov[4 * i + 2] * inv, ov[4 * i + 3] * inv);
+                __syncwarp();
             }
         }
-        named_bar_sync(1, kSoftmaxThreads);
-        for (int r = warp; r < kQTile; r += kSoftmaxThreads / 32) {
-            if (s0 + r < S) {
-                const float4 val = *reinterpret_cast<const float4 *>(&stage[r * kOutStride + 4 * lane]);
-                const long long o = (static_cast<long long>(s0 + r) * sh.H + h) * kD + 4 * lane;
-                if (out_f16) {
-                    *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(out) + o) = make_uint2(pack_half2(val.x, val.y), pack_half2(val.z, val.w));
-                } else {
-                    *reinterpret_cast<float4 *>(out + o) = val;
-                }
-            }
-        }
-        jt0 += n_kv;
-        if (pass + 1 < n_pass) {
-            tc_fence_before();
-            named_bar_sync(2, kThreads);   // pairs with the control warp: Q, K, V^T and the staging tile may be reused
-            tc_fence_after();
-        }
-      }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (warp == kMmaWarp) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
     if (sm.abort_flag && tid == 0) {
@@ -592,17 +798,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 
 }  // namespace
 
-// staging of one prefill call: f16 q [H][s_pad][D], then the cos/sin table f32 [2][S][32][2]
-static size_t prefill_q_bytes(int H, int S) {
-    const int s_pad = (S + kQTile - 1) / kQTile * kQTile;
-    return (static_cast<size_t>(H) * s_pad * kD * sizeof(__half) + 255) / 256 * 256;
-}
-size_t prefill_q_half_bytes(int H, int S) { return prefill_q_bytes(H, S) + static_cast<size_t>(2) * S * 32 * sizeof(float2); }
+// angle table of one call's sequence with explicit position ids (or an arena without a table): f32 [stream][token][32][2]
+size_t prefill_angle_bytes(int S) { return static_cast<size_t>(2) * S * 32 * sizeof(float2); }
 
-cudaError_t launch_prefill(const LaunchCtx &cx, const SeqDev &sq, const CUtensorMap &q_map, const CUtensorMap &k_map,
-                           const CUtensorMap &v_map, __half *q_half) {
-    const int S = sq.qlen;
-    const int s_pad = (S + kQTile - 1) / kQTile * kQTile;
+// tab: n_seq, seqs[].sq and v_map[] filled by the caller; k_map covers the whole arena.  own_angles: room for
+// prefill_angle_bytes of every sequence.
+cudaError_t launch_prefill(const LaunchCtx &cx, PrefillTable &tab, const CUtensorMap &k_map, float2 *own_angles) {
     static PerDeviceOnce configured;
     const int smem_bytes = static_cast<int>(sizeof(PrefillSmem)) + 1024;
     if (configured.needed(cx.device)) {
@@ -611,40 +812,57 @@ cudaError_t launch_prefill(const LaunchCtx &cx, const SeqDev &sq, const CUtensor
         if (e != cudaSuccess) return e;
         configured.mark(cx.device);
     }
-    // Angles: positions derived from the token index lie inside the arena's table (one row per cache position);
-    // explicit position ids may not, so a call that brings them gets a table of its own first.
-    const float2 *table = cx.rope_tab;
-    int table_by_position = 1;
-    int launched = 2;
-    if (rope_n_pairs_host(cx.shape.rope_type) > 0 && (sq.position_ids || !cx.rope_tab || S > cx.rope_tab_len)) {
-        float2 *own = reinterpret_cast<float2 *>(reinterpret_cast<uint8_t *>(q_half) + prefill_q_bytes(cx.shape.H, S));
-        const int n_entries = (cx.shape.rope_type == CGLM_ROPE_CHATGLM ? 2 : 1) * S * 32;
-        rope_table_kernel<<<(n_entries + 255) / 256, 256, 0, cx.stream>>>(cx.shape, sq, own);
-        table = own;
-        table_by_position = 0;
-        ++launched;
+    const AttnShape &sh = cx.shape;
+    int launched = 2, blocks = 0;
+    long long tiles = 0;
+    for (int i = 0; i < tab.n_seq; ++i) {
+        PrefillSeq &ps = tab.seqs[i];
+        const int S = ps.sq.qlen;
+        ps.n_q = (S + kQTile - 1) / kQTile;
+        ps.block_begin = blocks;
+        blocks += (S + kAppTokens - 1) / kAppTokens;
+        tiles += static_cast<long long>(ps.n_q) * sh.H;
+        ps.causal = ps.sq.n_past == 0 && sh.mask_type == CGLM_MASK_CAUSAL;
+        ps.blocked = ps.sq.n_past == 0 && sh.mask_type == CGLM_MASK_CHATGLM;
+        ps.vec = decode_rows_aligned(ps.sq.q, ps.sq.k, ps.sq.v, ps.sq.q_head_stride, ps.sq.kv_head_stride, nullptr, nullptr,
+                                     (ps.sq.flags & CGLM_SEQ_QKV_F16) != 0) &&
+                 ps.sq.q_tok_stride % 4 == 0 && ps.sq.kv_tok_stride % 4 == 0;
+        // Angles: positions derived from the token index lie inside the arena's table (one row per cache position);
+        // explicit position ids may not, so such a sequence gets a table of its own first.
+        ps.angles = cx.rope_tab;
+        ps.by_position = 1;
+        if (sh.rope_type != CGLM_ROPE_DISABLED && (ps.sq.position_ids || !cx.rope_tab || ps.sq.n_past + S > cx.rope_tab_len)) {
+            const int n_entries = (sh.rope_type == CGLM_ROPE_CHATGLM ? 2 : 1) * S * 32;
+            rope_table_kernel<<<(n_entries + 255) / 256, 256, 0, cx.stream>>>(sh, ps.sq, own_angles);
+            ps.angles = own_angles;
+            ps.by_position = 0;
+            own_angles += static_cast<size_t>(2) * S * 32;
+            ++launched;
+        }
+    }
+    // One tile per CTA while all tiles still run at once (a short prompt: more SMs, and nothing to overlap with); otherwise two.
+    tab.mode = tiles <= cx.n_sm ? kPrefillSingle : (sh.R > 1 ? kPrefillPairHeads : kPrefillPairTiles);
+    int units = 0;
+    for (int i = 0; i < tab.n_seq; ++i) {
+        PrefillSeq &ps = tab.seqs[i];
+        ps.unit_begin = units;
+        units += tab.mode == kPrefillSingle ? ps.n_q * sh.H : (tab.mode == kPrefillPairHeads ? ps.n_q * sh.G * ((sh.R + 1) / 2) : (ps.n_q + 1) / 2 * sh.H);
     }
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see griddepcontrol.wait in both kernels
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t pcfg = {};
-    pcfg.gridDim = dim3((S + kPrepTokens - 1) / kPrepTokens, (cx.shape.H + 1) / 2 + 2 * cx.shape.G);
-    pcfg.blockDim = dim3(kPrepThreads);
-    pcfg.stream = cx.stream;
-    pcfg.attrs = attr;
-    pcfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&pcfg, prefill_prepare_kernel, cx.shape, sq, cx.k_base, cx.v_base, q_half, s_pad, table,
-                                       table_by_position);
-    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((s_pad / kQTile + 1) / 2, cx.shape.H);   // each CTA takes q tiles (n_q - 1 - x) and x
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem_bytes;
+    cfg.gridDim = dim3(blocks, sh.G, 2);
+    cfg.blockDim = dim3(kAppThreads);
     cfg.stream = cx.stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, prefill_attn_kernel, q_map, k_map, v_map, cx.shape, S, sq.slot * cx.shape.G, sq.out,
-                           (sq.flags & CGLM_SEQ_OUT_F16) ? 1 : 0, cx.hdr);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, prefill_append_kernel, tab, sh, cx.k_base, cx.v_base);
+    if (e != cudaSuccess) return e;
+    cfg.gridDim = dim3(units < cx.n_sm ? units : (cx.n_sm < kPrefillMaxCtas ? cx.n_sm : kPrefillMaxCtas));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_bytes;
+    e = cudaLaunchKernelEx(&cfg, prefill_attn_kernel, k_map, tab, sh, units, cx.q_tiles, cx.hdr);
     g_launch_count += launched;
     return e != cudaSuccess ? e : cudaGetLastError();
 }

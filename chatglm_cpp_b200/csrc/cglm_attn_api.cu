@@ -34,6 +34,7 @@ struct cglm_kv_arena {
     size_t k_slot_elems;  // G*M*D
     bool has_tmaps;
     CUtensorMap k_map, v_map;
+    CUtensorMap k_map_prefill;  // the same K tensor in boxes of 64 dims x 128 tokens
     // pinned ring through which sequence descriptors travel to the device without a host sync
     SeqDev *ring;
     int ring_slots;
@@ -164,7 +165,7 @@ WsLayout ws_layout(const cglm_attn_desc &d, int n_sm, int n_seq, long long n_tok
     off = align_up(off + sizeof(SeqDev) * static_cast<size_t>(n_seq), 256);
     off = align_up(off, 1024);
     w.q_stage = off;
-    // roped, scaled q of the generic path (f32) or of one tcgen05 prefill (f16); used one launch at a time
+    // roped, scaled q of the generic path (f32), or the angle tables of tcgen05 prompts; used one launch at a time
     size_t stage = sizeof(float) * static_cast<size_t>(n_tokens) * d.n_head * d.head_dim;
     if (prefill_bytes > stage) stage = prefill_bytes;
     off = align_up(off + stage, 1024);
@@ -226,6 +227,11 @@ bool build_tensor_maps(cglm_kv_arena *a) {
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
+        box[1] = 128;
+        if (enc(&a->k_map_prefill, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, a->k_base, dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
     }
     {
         cuuint64_t dims[2] = {static_cast<cuuint64_t>(d.max_len), rows * d.head_dim};
@@ -240,40 +246,19 @@ bool build_tensor_maps(cglm_kv_arena *a) {
     return true;
 }
 
-// Per-call maps of the tcgen05 prefill: q staging f16 [H][s_pad][128]; the slot's K rows and V^T rows cut at the
-// attended length L, so that tokens past it read as zero whatever the cache holds there.
-bool build_prefill_maps(const cglm_kv_arena *a, void *q_half, int s_pad, int L, CUtensorMap *q_map, CUtensorMap *k_map,
-                        CUtensorMap *v_map) {
+// Per-sequence V^T map of the tcgen05 prompt path: cut at the attended length L, so that tokens past it read as zero whatever
+// the cache holds there (their probabilities are zero, but zero times an infinity is not).
+bool build_prefill_v_map(const cglm_kv_arena *a, int L, CUtensorMap *v_map) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return false;
     const cglm_attn_desc &d = a->desc;
     const cuuint64_t rows = static_cast<cuuint64_t>(a->n_slots) * d.n_kv_head;
-    const cuuint32_t estr3[3] = {1, 1, 1}, estr2[2] = {1, 1};
-    {
-        cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(s_pad), static_cast<cuuint64_t>(d.n_head)};
-        cuuint64_t strides[2] = {256, static_cast<cuuint64_t>(s_pad) * 256};
-        cuuint32_t box[3] = {64, 128, 1};
-        if (enc(q_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, q_half, dims, strides, box, estr3, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return false;
-    }
-    {
-        cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(L), rows};
-        cuuint64_t strides[2] = {256, static_cast<cuuint64_t>(d.max_len) * 256};
-        cuuint32_t box[3] = {64, 128, 1};
-        if (enc(k_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, a->k_base, dims, strides, box, estr3, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return false;
-    }
-    {
-        cuuint64_t dims[2] = {static_cast<cuuint64_t>(L), rows * 128};
-        cuuint64_t strides[1] = {static_cast<cuuint64_t>(d.max_len) * 2};
-        cuuint32_t box[2] = {64, 128};
-        if (enc(v_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a->v_base, dims, strides, box, estr2, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return false;
-    }
-    return true;
+    cuuint64_t dims[2] = {static_cast<cuuint64_t>(L), rows * 128};
+    cuuint64_t strides[1] = {static_cast<cuuint64_t>(d.max_len) * 2};
+    cuuint32_t box[2] = {64, 128};
+    const cuuint32_t estr[2] = {1, 1};
+    return enc(v_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a->v_base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 bool fast_decode_shape(const cglm_kv_arena *a) {
@@ -356,6 +341,8 @@ LaunchCtx make_launch_ctx(const cglm_kv_arena *a, uint8_t *ws, const WsLayout &l
     cx.partials = reinterpret_cast<float *>(ws + lay.partials);
     cx.gpartials = reinterpret_cast<float *>(ws + lay.gpartials);
     cx.q_stage = reinterpret_cast<float *>(ws + lay.q_stage);
+    cx.q_tiles = ws + sizeof(WsHeader);
+    static_assert(kLinearScratchBytes >= static_cast<size_t>(kPrefillMaxCtas) * 65536, "the prompt attention stages its q tiles there");
     cx.k_map = &a->k_map;
     cx.v_map = &a->v_map;
     cx.rope_tab = a->rope_tab;
@@ -602,8 +589,8 @@ size_t cglm_attn_workspace_bytes(const cglm_attn_desc *desc, int n_seq, int max_
     if (!desc_ok(desc) || n_seq <= 0 || max_qlen <= 0) return 0;
     int n_sm = 148, major = 0;
     device_sm_count(&n_sm, &major);   // falls back to a B200's SM count when no device is visible
-    // a prompt of >= 128 tokens at head_dim 128 may take the tensor-core prefill, whose staging is sized differently
-    const size_t prefill = desc->head_dim == 128 && max_qlen >= kPrefillMinTokens ? prefill_q_half_bytes(desc->n_head, max_qlen) : 0;
+    // prompts on the tensor-core path may need an angle table each
+    const size_t prefill = desc->head_dim == 128 && max_qlen >= kPrefillMinTokens ? n_seq * prefill_angle_bytes(max_qlen) : 0;
     return ws_layout(*desc, n_sm, n_seq, static_cast<long long>(n_seq) * max_qlen, prefill).total;
 }
 
@@ -705,11 +692,10 @@ int forward_impl(cglm_kv_arena *a, const cglm_attn_seq *seqs, int n_seq, void *w
         if (is_fast[i]) {
             ++n_fast;
             decode_tiles += static_cast<long long>((L + kDecodeTile - 1) / kDecodeTile) * d.n_kv_head;
-        } else if (prefill_ok && s.qlen >= kPrefillMinTokens && s.n_past == 0 && (s.flags & ~(CGLM_SEQ_CACHE_SETTLED | CGLM_SEQ_QKV_F16 | CGLM_SEQ_OUT_F16)) == 0) {
+        } else if (prefill_ok && s.qlen >= kPrefillMinTokens && (s.flags & ~(CGLM_SEQ_CACHE_SETTLED | CGLM_SEQ_QKV_F16 | CGLM_SEQ_OUT_F16)) == 0) {
             is_fast[i] = 2;
             ++n_prefill;
-            const size_t need = prefill_q_half_bytes(d.n_head, s.qlen);
-            if (need > prefill_bytes) prefill_bytes = need;
+            prefill_bytes += prefill_angle_bytes(s.qlen);
         } else {
             gen_tokens += s.qlen;
         }
@@ -774,21 +760,27 @@ int forward_impl(cglm_kv_arena *a, const cglm_attn_seq *seqs, int n_seq, void *w
             }
         }
     }
-    // generic path: descriptors are uploaded through the pinned ring
-    // tcgen05 prefill: one pair of launches per prompt, tensor maps encoded for this call
-    for (int i = 0; i < n_seq && n_prefill > 0; ++i) {
-        if (is_fast[i] != 2) continue;
-        SeqDev sq;
-        to_dev(seqs[i], sq);
-        const int s_pad = (sq.qlen + 127) / 128 * 128;
-        CUtensorMap q_map, k_map, v_map;
-        __half *q_half = reinterpret_cast<__half *>(ws + lay.q_stage);
-        if (!build_prefill_maps(a, q_half, s_pad, d.n_virtual + sq.qlen, &q_map, &k_map, &v_map)) {
-            std::snprintf(g_err, sizeof(g_err), "cuTensorMapEncodeTiled failed for a prefill call");
-            return CGLM_ERR_CUDA;
+    // tcgen05 prompts: kPrefillMaxSeq per pair of launches, the V^T tensor map of each encoded for this call
+    if (n_prefill > 0) {
+        static thread_local PrefillTable tab;
+        tab.n_seq = 0;
+        float2 *angles = reinterpret_cast<float2 *>(ws + lay.q_stage);
+        for (int i = 0, left = n_prefill; left > 0; ++i) {
+            if (is_fast[i] != 2) continue;
+            to_dev(seqs[i], tab.seqs[tab.n_seq].sq);
+            if (!build_prefill_v_map(a, tab.seqs[tab.n_seq].sq.kv_before + seqs[i].qlen, &tab.v_map[tab.n_seq])) {
+                std::snprintf(g_err, sizeof(g_err), "cuTensorMapEncodeTiled failed for a prefill call");
+                return CGLM_ERR_CUDA;
+            }
+            --left;
+            if (++tab.n_seq == kPrefillMaxSeq || left == 0) {
+                CGLM_CUDA(launch_prefill(cx, tab, a->k_map_prefill, angles));
+                for (int j = 0; j < tab.n_seq; ++j) angles += prefill_angle_bytes(tab.seqs[j].sq.qlen) / sizeof(float2);
+                tab.n_seq = 0;
+            }
         }
-        CGLM_CUDA(launch_prefill(cx, sq, q_map, k_map, v_map, q_half));
     }
+    // generic path: descriptors are uploaded through the pinned ring
     const int n_gen = n_seq - n_fast - n_prefill;
     if (n_gen > 0) {
         std::lock_guard<std::mutex> lock(a->mu);

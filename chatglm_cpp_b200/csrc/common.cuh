@@ -95,19 +95,38 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Returns false when the wait ran out (or an earlier wait of this CTA did): the caller carries on
-// without touching the barrier again.  *abort_flag lives in shared memory.
+// The same with a hint of how long the hardware may suspend the thread before it reports that the phase is still open.
+__device__ __forceinline__ bool mbar_try_wait_for(uint64_t *bar, uint32_t parity, uint32_t ns) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
+        : "memory");
+    return ok != 0;
+}
+// Returns false when the wait ran out (or this one is not met and an earlier wait of this CTA ran out): the caller carries
+// on without touching the barrier again.  *abort_flag lives in shared memory.  A waiting warp suspends in the barrier instead
+// of polling (polls take issue slots from the warps that work), so the wait is bounded by time: at most kWaitLimitNs.
+constexpr unsigned long long kWaitLimitNs = 1000000000ull;
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-    if (*abort_flag) {
-        return false;
+    if (mbar_try_wait(bar, parity)) {   // nothing else on the path of a wait that is already met
+        return true;
     }
+    unsigned long long t0 = 0;
     for (unsigned int i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) {
+        if (mbar_try_wait_for(bar, parity, 100000u)) {
             return true;
         }
-        if ((i & 1023u) == 1023u && *abort_flag) {
+        if (*abort_flag) {
             return false;
         }
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (t0 == 0) t0 = now;
+        if (now - t0 > kWaitLimitNs) break;
     }
     *abort_flag = 1;
     return false;
@@ -269,6 +288,7 @@ struct LaunchCtx {
     float *partials;             // decode split partials: 2 slots per CTA
     float *gpartials;            // decode group partials: 2 slots per group of 16 CTAs
     float *q_stage;              // generic path: roped, scaled q f32 [tokens][H][D]
+    uint8_t *q_tiles;            // prompt attention: two f16 q tiles per CTA (the Linear kernels' scratch region)
     const CUtensorMap *k_map;    // host copies of the arena's tensor maps (passed by value to kernels)
     const CUtensorMap *v_map;
     const float2 *rope_tab;      // arena's angle table: [rope_tab_len positions][32 ladder steps] (cos, sin); may be null
@@ -348,12 +368,30 @@ inline bool decode_rows_aligned(const float *q, const float *k, const float *v, 
     const uintptr_t out_bits = reinterpret_cast<uintptr_t>(q_roped) | reinterpret_cast<uintptr_t>(k_roped);
     return (in_bits & (qkv_f16 ? 7 : 15)) == 0 && (out_bits & 15) == 0 && q_head_stride % 4 == 0 && kv_head_stride % 4 == 0;
 }
-// tcgen05 prefill (head_dim 128, n_past == 0, qlen >= 128): per-call tensor maps over the f16 q staging buffer
-// [H][s_pad][D] and over the slot's caches cut at the attended length
-size_t prefill_q_half_bytes(int H, int S);
-cudaError_t launch_prefill(const LaunchCtx &cx, const SeqDev &sq, const CUtensorMap &q_map, const CUtensorMap &k_map,
-                           const CUtensorMap &v_map, __half *q_half);
-constexpr int kPrefillMinTokens = 128;
+// tcgen05 path of sequences with more than one token (head_dim 128): what the two launches know about up to kPrefillMaxSeq of
+// them, passed by value.  A sequence's V^T tensor map ends at its attended length.
+constexpr int kPrefillMaxSeq = 8;
+constexpr int kPrefillMaxCtas = 148;   // x 64 KiB of q tiles: what the Linear kernels' scratch holds
+enum { kPrefillSingle = 0, kPrefillPairHeads = 1, kPrefillPairTiles = 2 };   // q tiles per CTA, and which two
+struct PrefillSeq {
+    SeqDev sq;
+    const float2 *angles;   // arena's table (by_position) or this call's [stream][token][32]
+    int by_position;
+    int vec;                // q, k, v rows can be read four elements at a time
+    int causal, blocked;    // mask at n_past == 0: causal, or the v1 prefix mask
+    int n_q;                // 128-row tiles
+    int block_begin;        // first 64-token block of the append kernel
+    int unit_begin;         // first CTA of the attention kernel
+};
+struct PrefillTable {
+    CUtensorMap v_map[kPrefillMaxSeq];
+    PrefillSeq seqs[kPrefillMaxSeq];
+    int n_seq, mode;
+};
+size_t prefill_angle_bytes(int S);
+cudaError_t launch_prefill(const LaunchCtx &cx, PrefillTable &tab, const CUtensorMap &k_map, float2 *own_angles);
+// Shorter ones run on the generic path.
+constexpr int kPrefillMinTokens = 2;
 // fused query_key_value Linear + RoPE + append for one-token sequences (tcgen05): x_map f16 {64, n_tok, K/64} box
 // {64, qkv_linear_x_rows(n_tok), kb}, w_map f16 {64, n_feat, K/64} box {64, 32, kb}, both 128-byte swizzled;
 // kb (64-k blocks per box) <= qkv_linear_k_blocks(n_tok, K)
