@@ -29,11 +29,13 @@
 // the kernel and its first tile.
 // Both caches are already contraction-contiguous for the B operand: K is [token][d] for QK^T and V^T is
 // [d][token] for PV.
+#include <algorithm>
 #include <cstdlib>
 
 #include <type_traits>
 
 #include "common.cuh"
+#include "decode_rope.cuh"
 
 namespace cglm {
 
@@ -351,7 +353,6 @@ __device__ __forceinline__ void load_seq_desc(SeqDev &dst, const SeqDev &src, in
 //             inside the lane.
 //   CHATGLM:  each 64-dim half rotates as pairs (i, i+32) by ladder angle i, the first half by the position id and
 //             the second by the block position id: the partner of lane l sits in lane l ^ 8.
-__device__ __forceinline__ float4 ldg4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
 // four consecutive outputs at element index e of an f32 row, or of an f16 row with CGLM_SEQ_OUT_F16
 __device__ __forceinline__ void st_out4(float *row, long long e, bool f16, float a, float b, float c, float d) {
     if (f16) {
@@ -360,17 +361,6 @@ __device__ __forceinline__ void st_out4(float *row, long long e, bool f16, float
         *reinterpret_cast<float4 *>(row + e) = make_float4(a, b, c, d);
     }
 }
-__device__ __forceinline__ uint2 pack_half4(float a, float b, float c, float d) {
-    return make_uint2(pack_half2(a, b), pack_half2(c, d));
-}
-// Angle of a position the arena's table does not hold (explicit position ids beyond the cache capacity): out of
-// line, so that the double-precision sincos stays out of the instruction stream of the common case.
-__device__ __noinline__ float2 rope_angle_uncached(int pos, int i, float theta_scale) {
-    float2 cs;
-    rope_cos_sin(pos, i, theta_scale, cs.x, cs.y);
-    return cs;
-}
-
 __device__ __forceinline__ void prepare_segment(QBuf &qb, const AttnShape &sh, const SeqDev &sq, int g,
                                                 int row, bool has_last_tile, bool appender, int lane,
                                                 uint16_t *__restrict__ k_base, uint16_t *__restrict__ v_base,
@@ -435,46 +425,7 @@ __device__ __forceinline__ void prepare_segment(QBuf &qb, const AttnShape &sh, c
         __syncwarp();     // so that these few small loads do not queue behind 96 KiB of them
         if (lane == 0) mbar_arrive(loads_issued);
     }
-    // Rotation of the 17 rows, in place.  Every product and sum is rounded separately and in the order of
-    // rope_rotate(): y0 = x0 c - x1 s, y1 = x0 s + x1 c.
-    if (mode == CGLM_ROPE_CHATGLM2) {
-        // lanes 0..15 hold pairs 2l and 2l+1 entirely; lanes 16..31 hold dims that do not rotate
-        const int a = (2 * lane) & 31;
-        const float ca = __shfl_sync(0xffffffffu, cs0.x, a), sa = __shfl_sync(0xffffffffu, cs0.y, a);
-        const float cb = __shfl_sync(0xffffffffu, cs0.x, a + 1), sb = __shfl_sync(0xffffffffu, cs0.y, a + 1);
-        const bool rot = lane < 16;
-#pragma unroll
-        for (int r = 0; r <= kRows; ++r) {
-            float4 y;
-            rope_rotate(x[r].x, x[r].y, ca, sa, y.x, y.y);
-            rope_rotate(x[r].z, x[r].w, cb, sb, y.z, y.w);
-            if (rot) x[r] = y;
-        }
-    } else if (mode == CGLM_ROPE_CHATGLM) {
-        // lane l holds x_i (bit 3 of l clear) or x_{i+32} (set) of four pairs; the other element sits in lane l ^ 8
-        const bool second = lane >= 16, upper = (lane & 8) != 0;
-        float c[4], sg[4];   // sg: the sine with the sign this lane's element takes (-s for x_i, +s for x_{i+32})
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int a = 4 * (lane & 7) + e;
-            const float c0 = __shfl_sync(0xffffffffu, cs0.x, a), s0 = __shfl_sync(0xffffffffu, cs0.y, a);
-            const float c1 = __shfl_sync(0xffffffffu, cs1.x, a), s1 = __shfl_sync(0xffffffffu, cs1.y, a);
-            c[e] = second ? c1 : c0;
-            sg[e] = second ? s1 : s0;
-        }
-#pragma unroll
-        for (int r = 0; r <= kRows; ++r) {
-            const float ox = __shfl_xor_sync(0xffffffffu, x[r].x, 8), oy = __shfl_xor_sync(0xffffffffu, x[r].y, 8);
-            const float oz = __shfl_xor_sync(0xffffffffu, x[r].z, 8), ow = __shfl_xor_sync(0xffffffffu, x[r].w, 8);
-            // x_i:      y = x c - o s  (rope_rotate's y0 with x0 = x, x1 = o)
-            // x_{i+32}: y = o s + x c  (rope_rotate's y1 with x0 = o, x1 = x); the sum commutes exactly
-            const float px = __fmul_rn(ox, sg[0]), py = __fmul_rn(oy, sg[1]), pz = __fmul_rn(oz, sg[2]), pw = __fmul_rn(ow, sg[3]);
-            x[r].x = upper ? __fadd_rn(px, __fmul_rn(x[r].x, c[0])) : __fsub_rn(__fmul_rn(x[r].x, c[0]), px);
-            x[r].y = upper ? __fadd_rn(py, __fmul_rn(x[r].y, c[1])) : __fsub_rn(__fmul_rn(x[r].y, c[1]), py);
-            x[r].z = upper ? __fadd_rn(pz, __fmul_rn(x[r].z, c[2])) : __fsub_rn(__fmul_rn(x[r].z, c[2]), pz);
-            x[r].w = upper ? __fadd_rn(pw, __fmul_rn(x[r].w, c[3])) : __fsub_rn(__fmul_rn(x[r].w, c[3]), pw);
-        }
-    }
+    rope_rows<kRows + 1>(x, mode, lane, cs0, cs1);
     const bool want_q = has_last_tile && sq.q_roped != nullptr && !dry;
 #pragma unroll
     for (int r = 0; r < kRows; ++r) {
@@ -1015,14 +966,7 @@ decode_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__
                         for (int gi = 0; gi < 2; ++gi) {
                             const unsigned int *gp = tab.gate[gi];
                             if (!gp) continue;
-                            bool seen = false;
-                            for (unsigned int spin = 0; spin < kSpinLimit && !sm.abort_flag; ++spin) {
-                                unsigned int v;
-                                asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(gp) : "memory");
-                                if (v == tab.gate_value[gi]) { seen = true; break; }
-                                __nanosleep(200);
-                            }
-                            if (!seen) sm.abort_flag = 1;
+                            if (!wait_gate(gp, tab.gate_value[gi], &sm.abort_flag)) sm.abort_flag = 1;
                         }
                     }
                     __syncwarp();
@@ -1289,11 +1233,33 @@ decode_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__
 
 int decode_max_ctas(int n_sm) { return 2 * n_sm; }   // bound used to size scratch; launch_decode picks the grid
 
+// Thread blocks per cluster with which decode_cluster_kernel takes a launch, 0: the persistent kernel takes it.
+// Clusters of eight up to 8 items (sequences x kv heads), of four up to a quarter of the SMs, of two up to half of them: one
+// thread block per SM with room for the clusters' placement (16 clusters of eight do not fit the 148 SMs at once: 14.4 us per
+// launch against 7.4 for 8).  The line is the longest item, because an item cannot borrow another's warps: 8 tiles (512
+// tokens) per thread block.  Measured, us per launch in a chain, f16 activations, persistent kernel -> clusters:
+//   8 thread blocks, 1 / 4 sequences   512 tokens 10.5 -> 6.7 / 10.9 -> 7.4   2048 13.5 -> 10.1 / 20.3 -> 12.4   4096 17.6 -> 16.6 / 35.7 -> 19.0
+//   4 thread blocks, 16 sequences      512 tokens 22.9 -> 10.0   1024 25.2 -> 13.7   2048 28.5 -> 20.5   4096 27.1 -> 28.2
+//   2 thread blocks, 32 sequences      512 tokens 21.5 -> 13.6   1024 25.2 -> 20.4   2048 27.4 -> 28.4
+//   one q head per kv head, 32 of them: 2048 tokens 20.2 -> 19.3 with 4, two sequences 1024 tokens 21.3 -> 19.1 with 2
+int decode_cluster_ctas(const DecodeTable &tab, int G, int n_sm) {
+    const int n_items = tab.n_seq * G;
+    if (tab.n_seq > kDecodeClusterMaxSeq || 2 * n_items > n_sm) return 0;
+    const int n_cta = n_items <= 8 ? 8 : (4 * n_items <= n_sm ? 4 : 2);
+    int longest = 0;
+    for (int i = 0; i < tab.n_seq; ++i) longest = std::max(longest, tab.prefix[i + 1] - tab.prefix[i]);
+    return longest <= 8 * n_cta ? n_cta : 0;
+}
+
 cudaError_t launch_decode(const LaunchCtx &cx, const DecodeTableDyn &tab, bool n_past_on_device, const XchgDev *xchg) {
     // with device-side positions tab.prefix holds the tile counts of the host's upper bounds: good for sizing only
     const long long total_tiles = static_cast<long long>(tab.prefix[tab.n_seq]) * cx.shape.G;
     if (tab.n_seq == 0 || total_tiles == 0) {
         return cudaSuccess;
+    }
+    if (!xchg) {
+        const int n_cta = decode_cluster_ctas(tab, cx.shape.G, cx.n_sm);
+        if (n_cta > 0) return launch_decode_cluster(cx, tab, n_cta);
     }
     static PerDeviceOnce configured;
     const int smem_bytes = static_cast<int>(sizeof(DecodeSmem)) + 1024;

@@ -149,8 +149,7 @@ struct WsLayout {
 WsLayout ws_layout(const cglm_attn_desc &d, int n_sm, int n_seq, long long n_tokens, size_t prefill_bytes = 0) {
     WsLayout w;
     size_t off = sizeof(WsHeader);
-    // scratch of the Linear kernels (partial sums of k-split tiles), at a fixed offset so that cglm_linear_forward finds
-    // it in any workspace without knowing the attention configuration
+    // q tiles of long prompts (PrefillTable), the room that every workspace also offers the Linears
     off = align_up(off + kLinearScratchBytes, 256);
     w.counters = off;
     off = align_up(off + sizeof(int) * kDecodeMaxSeqPerLaunch * static_cast<size_t>(d.n_kv_head), 256);
@@ -1093,7 +1092,7 @@ int try_linear_fm(int device, int n_sm, cudaStream_t st, const LaunchCtx *qkv_cx
     if (tokens_on_m || workspace_bytes < sizeof(WsHeader) + kLinearScratchBytes) return 1;
     if (reinterpret_cast<uintptr_t>(bias) & 15) return 1;   // this kernel reads the bias four features at a time
     LinearFmPlan plan;
-    if (!linear_fm_plan(n_tok, K, n_feat, n_sm, kLinearScratchBytes, &plan)) return 1;
+    if (!linear_fm_plan(n_tok, K, n_feat, n_sm, &plan)) return 1;
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return CGLM_ERR_CUDA;
     CUtensorMap x_map, w_map;
@@ -1108,8 +1107,7 @@ int try_linear_fm(int device, int n_sm, cudaStream_t st, const LaunchCtx *qkv_cx
         cx.n_sm = n_sm;
         cx.device = device;
     }
-    float *scratch = reinterpret_cast<float *>(static_cast<uint8_t *>(workspace) + sizeof(WsHeader));
-    CGLM_CUDA(launch_linear_fm(cx, plan, x_map, w_map, slots, n_past, n_tok, K, n_feat, bias, q_out, out, out_f16, scratch));
+    CGLM_CUDA(launch_linear_fm(cx, plan, x_map, w_map, slots, n_past, n_tok, K, n_feat, bias, q_out, out, out_f16, weight_f16));
     return CGLM_OK;
 }
 
@@ -1120,7 +1118,7 @@ size_t cglm_linear_workspace_bytes(void) { return sizeof(WsHeader) + kLinearScra
 int cglm_linear_kernel_plan(int n_tok, int in_features, int out_features, int n_sm, int plan[8]) {
     if (!plan || n_sm <= 0) return 0;
     LinearFmPlan p;
-    if (!linear_fm_plan(n_tok, in_features, out_features, n_sm, kLinearScratchBytes, &p)) return 0;
+    if (!linear_fm_plan(n_tok, in_features, out_features, n_sm, &p)) return 0;
     plan[0] = p.n_box; plan[1] = p.tiles; plan[2] = p.token_tiles; plan[3] = p.ksplit;
     plan[4] = p.blocks_per_cta; plan[5] = p.kb; plan[6] = p.n_stages; plan[7] = p.tmem_cols;
     return 1;

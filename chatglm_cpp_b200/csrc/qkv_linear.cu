@@ -294,15 +294,30 @@ qkv_linear_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
 // and every CTA pulls all of x through L2 (512 KB for 64 tokens, twice its slice of the weight).  Here a CTA owns 128
 // output features (the M rows; one head of a head_dim-128 model) and the tokens are the N columns (16 .. 128), so an
 // MMA reads 4 KB of weight and 32 bytes per token.  128 features per CTA are only n_feat / 128 tiles (36 for a GLM-4
-// query_key_value), too few CTAs to pull the weight from HBM, so the k range is split over `ksplit` CTAs per tile
-// (36 x 4 = 144 CTAs): each writes its partial sums [token][128 features] to scratch in the workspace, the last one to
-// arrive at the tile's counter adds the partials in split order (the same bits whatever the arrival order) and runs the
-// epilogue.  Without a split (prompts: tiles x token tiles fill the GPU) the sums pass through shared memory instead.
-// No CTA waits for another: the counter decides who finishes the tile.
+// query_key_value), too few CTAs to pull the weight from HBM, so the k range is split over the `ksplit` CTAs of a cluster
+// (36 x 4 = 144 CTAs): each leaves its partial sums [token][128 features] in its own shared memory, and after a cluster
+// barrier every CTA adds up its share of the tile from all of them, in split order (the same bits whichever CTA comes
+// first), and runs the epilogue on it.
+//
+// What bounds a decode-sized launch is the chain of kernels around it, not its own traffic: the weight takes 5 us of HBM
+// time, and none of it depends on the kernel in front.  So a split launch is kept small enough (kFmSplitSmem) to come up
+// beside the CTAs of that kernel, fills its ring with weights and asks for the rest of its slice in L2 before its
+// dependency wait.
+//
+// Measured (per replay of a 28-layer step of one 512-token chat, every layer's own weights, with decode_cluster_kernel between
+// the Linears): with the partial sums through L2, a counter and all of an SM's shared memory 1020 us, as it is now 815 us; 64
+// sequences x 4 layers 371 -> 365 us.
 constexpr int kFmFeat = 128;                 // M of the MMA: output features per CTA
 constexpr int kFmWBytes = kFmFeat * 128;     // W tile of one 64-k block: [128 features][64 k] f16
 constexpr int kFmMaxStages = 8;
-constexpr int kFmBatch = 6;                  // (token, 4 features) items a thread has in flight in the finishing pass
+// (token, 4 features) items a thread has in flight in the finishing pass: up to 64 tokens are one batch
+constexpr int fm_batch(int ksplit) { return ksplit == 4 ? 3 : 6; }
+// Shared memory of a CTA of a split launch: two such CTAs, or one beside a CTA of the decode kernel (at most this much as
+// well), fit the 228 KiB of an SM with 1 KiB reserved for each.
+constexpr int kFmSplitSmem = 112640;
+// The requests into L2 leave this much after the ring's: at once they stand in front of what the previous kernel still has to
+// load (829 us per step with no delay, 824 / 815 / 813 with 1 / 2 / 3.5 us).
+constexpr unsigned int kFmPrefetchDelayNs = 2000;
 
 struct __align__(1024) FmSmem {
     uint64_t full[kFmMaxStages];
@@ -310,9 +325,8 @@ struct __align__(1024) FmSmem {
     uint64_t acc_full;
     uint32_t tmem_base;
     int abort_flag;
-    int is_last;
-    // 1024-byte aligned: n_stages stages of (kb x tiles of n_box token rows | kb W tiles); after the last MMA the sums
-    // [token][128] of an unsplit tile
+    // 1024-byte aligned: n_stages stages of (kb x tiles of n_box token rows | kb W tiles); after the last MMA this CTA's
+    // sums [token][128]
     __align__(1024) uint8_t ring[1];
 };
 
@@ -323,9 +337,8 @@ struct FmArgs {
     int blocks_per_cta;   // 64-k blocks one CTA sums over: K / 64 / ksplit
     int ksplit;
     int tmem_cols;        // power of two >= max(n_box, 32)
+    const uint16_t *w;    // the weight [n_feat][K], for the prefetch of a split launch
     const float *bias;
-    float *scratch;       // ksplit > 1: partial sums [tile][split][n_box][128]
-    int *tile_counters;   // ksplit > 1: arrivals per (token tile, feature tile), self-resetting
     WsHeader *hdr;
     void *out;            // plain epilogue: f32 or f16 [n_tok][n_feat]
     int out_f16;
@@ -334,6 +347,10 @@ struct FmArgs {
     const float2 *rope_tab;
     int rope_tab_len;
 };
+
+__device__ __forceinline__ void cluster_sync() {   // every thread of the cluster, and its memory operations
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 template <bool kPlain>
 __device__ __forceinline__ void fm_finish_item(const FmArgs &a, const QkvTable &tab, const AttnShape &sh, int f0, int tok, int q, float4 v) {
@@ -389,13 +406,20 @@ __device__ __forceinline__ void fm_finish_item(const FmArgs &a, const QkvTable &
     }
 }
 
-// Finishing pass of one tile by all threads of the CTA: item = (token, 4 consecutive features).  Every load of a batch of
-// items (all splits) is issued before the first sum, so that a thread waits for L2 once per batch, not once per split;
-// the splits are added in order, whoever arrived last.
+// Finishing pass of items [first, last) of one tile by all threads of the CTA: item = (token, 4 consecutive features).
+// sums: shared address of the CTA's own sums, at which the other CTAs of the cluster hold theirs too.  Every load of a
+// batch of items (all splits) is issued before the first sum; the splits are added in order.
 template <bool kPlain, int kSplit>
-__device__ __forceinline__ void fm_finish_tile(const FmArgs &a, const QkvTable &tab, const AttnShape &sh, const float *part0,
-                                               size_t split_stride, int n_items, int f0, int tok0, int tid) {
-    for (int base = tid; base < n_items; base += kThreads * kFmBatch) {
+__device__ __forceinline__ void fm_finish_tile(const FmArgs &a, const QkvTable &tab, const AttnShape &sh, uint32_t sums,
+                                               int first, int last, int f0, int tok0, int tid) {
+    uint32_t src[kSplit];
+#pragma unroll
+    for (int s = 0; s < kSplit; ++s) {
+        src[s] = sums;
+        if (kSplit > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(src[s]) : "r"(sums), "r"(s));
+    }
+    constexpr int kFmBatch = fm_batch(kSplit);
+    for (int base = first + tid; base < last; base += kThreads * kFmBatch) {
         float4 v[kFmBatch][kSplit];
 #pragma unroll
         for (int u = 0; u < kFmBatch; ++u) {
@@ -403,9 +427,15 @@ __device__ __forceinline__ void fm_finish_tile(const FmArgs &a, const QkvTable &
 #pragma unroll
             for (int s = 0; s < kSplit; ++s) {
                 v[u][s] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (idx < n_items) {
-                    const float4 *src = reinterpret_cast<const float4 *>(part0 + s * split_stride) + idx;
-                    v[u][s] = kSplit > 1 ? __ldcg(src) : *src;
+                if (idx < last) {
+                    const uint32_t at = src[s] + static_cast<uint32_t>(idx) * 16u;
+                    if constexpr (kSplit > 1) {
+                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(v[u][s].x), "=f"(v[u][s].y), "=f"(v[u][s].z), "=f"(v[u][s].w) : "r"(at) : "memory");
+                    } else {
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(v[u][s].x), "=f"(v[u][s].y), "=f"(v[u][s].z), "=f"(v[u][s].w) : "r"(at) : "memory");
+                    }
                 }
             }
         }
@@ -418,13 +448,14 @@ __device__ __forceinline__ void fm_finish_tile(const FmArgs &a, const QkvTable &
                 t.x = __fadd_rn(t.x, v[u][s].x); t.y = __fadd_rn(t.y, v[u][s].y);
                 t.z = __fadd_rn(t.z, v[u][s].z); t.w = __fadd_rn(t.w, v[u][s].w);
             }
-            if (idx < n_items) fm_finish_item<kPlain>(a, tab, sh, f0, tok0 + (idx >> 5), idx & 31, t);
+            if (idx < last) fm_finish_item<kPlain>(a, tab, sh, f0, tok0 + (idx >> 5), idx & 31, t);
         }
     }
 }
 
 template <bool kPlain>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(256, 2)   // 128 registers: two of the six warps share a quarter of an SM's registers with
+                                            // a warp of decode_cluster_kernel
 linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map,
                  const __grid_constant__ QkvTable tab, const __grid_constant__ FmArgs a, AttnShape sh) {
     extern __shared__ uint8_t smem_raw[];
@@ -442,7 +473,6 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
 
     if (tid == 0) {
         sm.abort_flag = 0;
-        sm.is_last = 1;
         for (int s = 0; s < n_stages; ++s) {
             mbar_init(&sm.full[s], 1);
             mbar_init(&sm.empty[s], 1);
@@ -458,13 +488,11 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sm.tmem_base;
-    // x, the scratch and the outputs may still be in use by the previous kernel: only the weights are touched before it
-    // has completed (the first round of the ring is filled with them ahead of the wait)
+    // x and the outputs may still be in use by the previous kernel: only the weights are touched before it has completed
+    // (the first round of the ring is filled with them ahead of the wait)
 
     if (warp == kTmaWarp) {
         if (lane == 0) {
-            tma_prefetch_desc(&x_map);
-            tma_prefetch_desc(&w_map);
             const int pre = n_stages < n_k ? n_stages : n_k;
             for (int i = 0; i < pre; ++i) {
                 mbar_arrive_expect_tx(&sm.full[i], stage_bytes);
@@ -505,12 +533,16 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         }
     } else {
         // ===== warps 0..3: TMEM lane t = feature f0 + t, column j = token j; hand the sums on as [token][128] ==========
-        asm volatile("griddepcontrol.wait;" ::: "memory");   // before this thread writes the scratch
+        if (a.ksplit > 1 && n_k > n_stages) {
+            // what the ring does not hold of weight row f0 + tid (its k are contiguous): into L2 while the previous kernel runs
+            const long long k0 = static_cast<long long>(k_base + n_stages * kb) * kKStep;
+            const uint32_t bytes = static_cast<uint32_t>((n_k - n_stages) * kb) * 128u;
+            __nanosleep(kFmPrefetchDelayNs);
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.w + static_cast<long long>(f0 + tid) * a.K + k0), "r"(bytes) : "memory");
+        }
         mbar_wait_bounded(&sm.acc_full, 0, &sm.abort_flag);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        float *dump = a.ksplit > 1
-                          ? a.scratch + (static_cast<size_t>(ttile * gridDim.x + tile) * a.ksplit + split) * a.n_box * kFmFeat
-                          : reinterpret_cast<float *>(sm.ring);
+        float *dump = reinterpret_cast<float *>(sm.ring);
         const uint32_t taddr = tmem + (static_cast<uint32_t>(32 * warp) << 16);
         for (int c = 0; c < n_real; c += 16) {   // the same trip count in every thread
             uint32_t r[16];
@@ -522,33 +554,29 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
                 : "r"(taddr + static_cast<uint32_t>(c))
                 : "memory");
 #pragma unroll
-            for (int j = 0; j < 16; ++j) dump[(c + j) * kFmFeat + tid] = __uint_as_float(r[j]);   // rows < n_box: inside the block
+            for (int j = 0; j < 16; ++j) dump[(c + j) * kFmFeat + tid] = __uint_as_float(r[j]);   // rows < n_box: inside the ring
         }
-        if (a.ksplit > 1) __threadfence();
     }
+    __syncwarp();   // the cluster barrier below wants whole warps
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    // every thread that writes an output has seen the previous kernel complete
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int n_items = n_real * (kFmFeat / 4);
+    const uint32_t sums = smem_u32(sm.ring);
     if (a.ksplit > 1) {
-        if (tid == 0) {
-            int *counter = a.tile_counters + ttile * gridDim.x + tile;
-            const int last = atomicAdd(counter, 1) == a.ksplit - 1;
-            if (last) *counter = 0;   // for the next launch; nobody else touches it any more
-            sm.is_last = last;
+        // all sums of the tile are in the cluster's shared memory; a CTA finishes every ksplit-th part of the items.  The
+        // second barrier keeps a CTA's shared memory alive until its peers have read it.
+        cluster_sync();
+        const int first = n_items * split / a.ksplit, last = sm.abort_flag ? 0 : n_items * (split + 1) / a.ksplit;
+        if (a.ksplit == 4) {
+            fm_finish_tile<kPlain, 4>(a, tab, sh, sums, first, last, f0, tok0, tid);
+        } else {
+            fm_finish_tile<kPlain, 2>(a, tab, sh, sums, first, last, f0, tok0, tid);
         }
+        cluster_sync();
+    } else {
         __syncthreads();
-    }
-    if (sm.is_last && !sm.abort_flag) {
-        if (a.ksplit > 1) __threadfence();
-        // ===== all six warps: sum the splits in order, bias, epilogue; item = (token, 4 consecutive features) ===========
-        const int n_items = n_real * (kFmFeat / 4);
-        const size_t split_stride = static_cast<size_t>(a.n_box) * kFmFeat;
-        const float *part0 = a.ksplit > 1 ? a.scratch + static_cast<size_t>(ttile * gridDim.x + tile) * a.ksplit * split_stride
-                                          : reinterpret_cast<const float *>(sm.ring);
-        switch (a.ksplit) {
-        case 4: fm_finish_tile<kPlain, 4>(a, tab, sh, part0, split_stride, n_items, f0, tok0, tid); break;
-        case 2: fm_finish_tile<kPlain, 2>(a, tab, sh, part0, split_stride, n_items, f0, tok0, tid); break;
-        default: fm_finish_tile<kPlain, 1>(a, tab, sh, part0, split_stride, n_items, f0, tok0, tid); break;
-        }
+        fm_finish_tile<kPlain, 1>(a, tab, sh, sums, 0, sm.abort_flag ? 0 : n_items, f0, tok0, tid);
     }
     __syncthreads();
     if (warp == 0) {
@@ -648,29 +676,32 @@ cudaError_t launch_linear_plain(int device, cudaStream_t stream, WsHeader *hdr, 
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+constexpr int fm_sum_bytes(int n_box) { return n_box * kFmFeat * static_cast<int>(sizeof(float)); }
+static_assert(2048 + fm_sum_bytes(128) <= kFmSplitSmem, "the sums of a split launch fit in the place of its ring");
+
 // ---- features on the M side: plan and launch -------------------------------------------------------------------------
-bool linear_fm_plan(int n_tok, int K, int n_feat, int n_sm, size_t scratch_bytes, LinearFmPlan *p) {
+bool linear_fm_plan(int n_tok, int K, int n_feat, int n_sm, LinearFmPlan *p) {
     if (n_tok <= 0 || K % kKStep != 0 || n_feat % kFmFeat != 0) return false;
     const int tiles = n_feat / kFmFeat, ttiles = (n_tok + 127) / 128;
     p->n_box = n_tok > 128 ? 128 : (n_tok + 15) / 16 * 16;
     p->tiles = tiles;
     p->token_tiles = ttiles;
-    // split k while the CTAs of all tiles still run at once; a split tile needs a counter in the workspace header and
-    // scratch for its partial sums
+    // split k while the CTAs of all tiles still run at once
     p->ksplit = 1;
     for (int sp = 4; sp >= 2; sp >>= 1) {
         const long long ctas = static_cast<long long>(tiles) * ttiles * sp;
-        if (ctas <= n_sm && (K / kKStep) % sp == 0 && tiles * ttiles <= kLinearFmMaxSplitTiles &&
-            static_cast<size_t>(ctas) * p->n_box * kFmFeat * sizeof(float) <= scratch_bytes) {
+        if (ctas <= n_sm && (K / kKStep) % sp == 0 && tiles * ttiles <= kLinearFmMaxSplitTiles) {
             p->ksplit = sp;
             break;
         }
     }
     p->blocks_per_cta = K / kKStep / p->ksplit;
-    const int ring = kSmemPerCta - 2048;
+    // an unsplit launch has an SM to itself and does best with large boxes and two stages; a split one is smaller and keeps
+    // three boxes in flight (its sums are 64 KiB at most, less than any ring of three)
+    const int ring = (p->ksplit > 1 ? kFmSplitSmem : kSmemPerCta) - 2048;
     p->kb = 1;
     for (int kb = 4; kb > 1; kb >>= 1) {
-        if (p->blocks_per_cta % kb == 0 && ring / (kb * (p->n_box * 128 + kFmWBytes)) >= 2) {
+        if (p->blocks_per_cta % kb == 0 && ring / (kb * (p->n_box * 128 + kFmWBytes)) >= (p->ksplit > 1 ? 3 : 2)) {
             p->kb = kb;
             break;
         }
@@ -682,8 +713,8 @@ bool linear_fm_plan(int n_tok, int K, int n_feat, int n_sm, size_t scratch_bytes
     if (n_stages < 1) return false;
     p->n_stages = n_stages;
     p->tmem_cols = p->n_box <= 32 ? 32 : (p->n_box <= 64 ? 64 : 128);
-    // an unsplit tile hands its sums [n_box][128] f32 through the ring
-    if (p->ksplit == 1 && n_stages * stage_bytes < p->n_box * kFmFeat * static_cast<int>(sizeof(float))) return false;
+    // an unsplit tile hands its sums [n_box][128] f32 through the ring (a split launch has room for them in any case)
+    if (p->ksplit == 1 && n_stages * stage_bytes < fm_sum_bytes(p->n_box)) return false;
     return true;
 }
 
@@ -691,7 +722,7 @@ bool linear_fm_plan(int n_tok, int K, int n_feat, int n_sm, size_t scratch_bytes
 // 128-byte swizzled.  slots / n_past non-null: query_key_value epilogue (q_out, caches of cx); null: plain (out).
 cudaError_t launch_linear_fm(const LaunchCtx &cx, const LinearFmPlan &plan, const CUtensorMap &x_map, const CUtensorMap &w_map,
                              const int *slots, const int *n_past, int n_tok, int K, int n_feat, const float *bias, float *q_out,
-                             void *out, bool out_f16, float *scratch) {
+                             void *out, bool out_f16, const void *weight_f16) {
     cudaError_t e = configure_once(cx.device);
     if (e != cudaSuccess) return e;
     static_assert(offsetof(FmSmem, ring) == 1024, "header, then the ring");
@@ -705,22 +736,24 @@ cudaError_t launch_linear_fm(const LaunchCtx &cx, const LinearFmPlan &plan, cons
     a.n_box = plan.n_box; a.kb = plan.kb; a.n_stages = plan.n_stages; a.blocks_per_cta = plan.blocks_per_cta;
     a.ksplit = plan.ksplit; a.tmem_cols = plan.tmem_cols;
     a.bias = bias;
-    a.scratch = scratch;
-    a.tile_counters = cx.hdr->reserved;
+    a.w = static_cast<const uint16_t *>(weight_f16);
     a.hdr = cx.hdr;
     a.out = out; a.out_f16 = out_f16 ? 1 : 0;
     a.q_out = q_out; a.k_base = cx.k_base; a.v_base = cx.v_base; a.rope_tab = cx.rope_tab; a.rope_tab_len = cx.rope_tab_len;
-    const int smem_bytes = 2048 + plan.n_stages * plan.kb * (plan.n_box * 128 + kFmWBytes);
-    cudaLaunchAttribute attr[1];
+    const int ring_bytes = plan.n_stages * plan.kb * (plan.n_box * 128 + kFmWBytes);
+    const int smem_bytes = 2048 + (ring_bytes > fm_sum_bytes(plan.n_box) ? ring_bytes : fm_sum_bytes(plan.n_box));
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = static_cast<unsigned>(plan.ksplit); attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.tiles, plan.ksplit, plan.token_tiles);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = cx.stream;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = plan.ksplit > 1 ? 2 : 1;
     if (slots) {
         e = cudaLaunchKernelEx(&cfg, linear_fm_kernel<false>, x_map, w_map, tab, a, cx.shape);
     } else {

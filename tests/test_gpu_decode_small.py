@@ -1,0 +1,50 @@
+"""Small decode launches (one thread-block cluster per sequence and kv head) against the CPU oracle, at the sizes where the split
+of an item over the cluster's warps can go wrong: one token, around a warp's 32 and a thread block's 128 tokens, around a whole
+round of the cluster (4 x 32 tokens per thread block), the capacity's last row; every cluster size the rule picks, and the lengths
+on both sides of its line.  Bounds: those of run_decode_batch (output within assert_out_close, caches bit-exact, roped rows 2 ulp)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import attn_oracle as O
+
+from gpu_util import assert_out_close, make_desc, oracle_cfg, qkv_width, random_cache, run_decode_batch, upload_cache
+
+pytestmark = pytest.mark.gpu
+
+ROUND = 1024   # tokens of one round of eight thread blocks
+LENS8 = [0, 1, 30, 31, 32, 127, 128, 129]
+
+
+@pytest.mark.parametrize("H,G,rope,mask,V,M,lens", [
+    (32, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 4160, [ROUND - 1]),                       # clusters of eight
+    (32, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 4160, [ROUND, 2 * ROUND + 33, 0, 4095]),   # the rule's line: 64 tiles of 64 tokens
+    (32, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 4160, [4096]),                             # just past it: the persistent kernel
+    (32, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 1096, LENS8 + [1095]),                     # clusters of four; the last cache row
+    (6, 2, O.ROPE_DISABLED, O.MASK_CAUSAL, 0, 520, LENS8),                                # three q heads per kv head
+    (32, 32, O.ROPE_CHATGLM, O.MASK_CHATGLM, 0, 1096, [700, 1023]),                       # clusters of two, one q head each
+    (4, 4, O.ROPE_CHATGLM, O.MASK_CHATGLM, 5, 520, LENS8),                                # a P-Tuning prefix
+])
+@pytest.mark.parametrize("on_device", [False, True])
+def test_small_decode(H, G, rope, mask, V, M, lens, on_device):
+    inter = rope == O.ROPE_CHATGLM
+    run_decode_batch(make_desc(H, G, 128, M, V, rope, 10000.0, mask), lens, seed=len(lens), interleaved=inter,
+                     n_ctx_list=[max(2, p // 2) for p in lens] if inter else None, n_past_on_device=on_device, f16_io=len(lens) > 4)
+
+
+def test_stale_cache_rows_behind_the_appended_token_do_not_reach_the_result():
+    """NaN in every cache row past the attended length: what the last chunk loads beside the item's own tokens."""
+    from chatglm_cpp_b200 import attention as A
+    desc = make_desc(16, 1, 128, 264)
+    rng = np.random.default_rng(5)
+    for P in (0, 7, 31, 64, 200):
+        arena, ws = A.KVArena(desc, 1), A.Workspace(desc, 1, 1)
+        k, v = random_cache(rng, desc, P)
+        k[:, P:], v[:, :, P:] = 0x7E00, 0x7E00
+        upload_cache(arena, 0, k, v)
+        qkv = rng.standard_normal((1, qkv_width(desc, False))).astype(np.float32)
+        out = A.BasicAttention(arena, 0, ws).forward(torch.from_numpy(qkv).cuda(), P)
+        torch.cuda.synchronize()
+        k[:, P:], v[:, :, P:] = 0, 0
+        assert_out_close(out.cpu().numpy(), O.attn_forward(oracle_cfg(desc, "f32"), qkv, False, k, v, P), f"n_past {P}")
+        arena.close()
