@@ -540,6 +540,7 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             __nanosleep(kFmPrefetchDelayNs);
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.w + static_cast<long long>(f0 + tid) * a.K + k0), "r"(bytes) : "memory");
         }
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // the bounded wait counts only time this grid could make progress
         mbar_wait_bounded(&sm.acc_full, 0, &sm.abort_flag);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         float *dump = reinterpret_cast<float *>(sm.ring);
@@ -565,7 +566,8 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     const uint32_t sums = smem_u32(sm.ring);
     if (a.ksplit > 1) {
         // all sums of the tile are in the cluster's shared memory; a CTA finishes every ksplit-th part of the items.  The
-        // second barrier keeps a CTA's shared memory alive until its peers have read it.
+        // second barrier keeps a CTA's shared memory alive until its peers have read it (what they read is in registers by
+        // then: nothing to order, and the output stores are not waited for).
         cluster_sync();
         const int first = n_items * split / a.ksplit, last = sm.abort_flag ? 0 : n_items * (split + 1) / a.ksplit;
         if (a.ksplit == 4) {
@@ -573,7 +575,8 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         } else {
             fm_finish_tile<kPlain, 2>(a, tab, sh, sums, first, last, f0, tok0, tid);
         }
-        cluster_sync();
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     } else {
         __syncthreads();
         fm_finish_tile<kPlain, 1>(a, tab, sh, sums, 0, sm.abort_flag ? 0 : n_items, f0, tok0, tid);
