@@ -48,3 +48,33 @@ def test_stale_cache_rows_behind_the_appended_token_do_not_reach_the_result():
         k[:, P:], v[:, :, P:] = 0, 0
         assert_out_close(out.cpu().numpy(), O.attn_forward(oracle_cfg(desc, "f32"), qkv, False, k, v, P), f"n_past {P}")
         arena.close()
+
+
+@pytest.mark.parametrize("G", [8, 10, 13, 16, 20])
+def test_merge_of_items_cut_into_many_parts(G):
+    """One sequence just past the clusters' line, cut over one thread block per SM: 7 to 18 parts per item, i.e. fewer than one
+    batch of copies, both of its barriers, more parts than slots in the tile ring, and the two-level merge."""
+    run_decode_batch(make_desc(2 * G, G, 128, 4168, 0, O.ROPE_CHATGLM2, 10000.0, O.MASK_CAUSAL), [4150], seed=G)
+
+
+@pytest.mark.parametrize("n_tok,n_in,n_out", [(128, 256, 128), (128, 512, 4096), (33, 4096, 4608), (1, 128, 128), (17, 4160, 256)])
+def test_linear_k_split_over_a_cluster(n_tok, n_in, n_out):
+    """Fewer weight blocks than the sums need room, one block per thread block, token counts that no CTA's share divides, a k that
+    four does and does not split evenly.  Bound: f32 sums of n_in products of f16 values, 2^-24 * sqrt(n_in) of the sum of their
+    sizes with a factor of 8."""
+    from chatglm_cpp_b200 import _lib
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n_tok + n_in)
+    x = torch.randn(n_tok, n_in, device="cuda", generator=gen).half()
+    w = torch.randn(n_out, n_in, device="cuda", generator=gen).half()
+    b = torch.randn(n_out, device="cuda", generator=gen)
+    L = _lib.lib()
+    ws = torch.zeros(L.cglm_linear_workspace_bytes(), dtype=torch.uint8, device="cuda")
+    out = torch.empty(n_tok, n_out, device="cuda")
+    torch.cuda.synchronize()
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(L.cglm_linear_forward(x.data_ptr(), n_tok, n_in, w.data_ptr(), n_out, b.data_ptr(), out.data_ptr(), 0, ws.data_ptr(),
+                                     ws.numel(), stream), "cglm_linear_forward")
+    want = x.double() @ w.double().T + b.double()
+    size = x.double().abs() @ w.double().abs().T + b.double().abs()
+    assert ((out.double() - want).abs() <= 8 * 2.0 ** -24 * n_in ** 0.5 * size).all()
