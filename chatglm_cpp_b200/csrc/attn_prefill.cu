@@ -1,7 +1,7 @@
 // Prompt attention on 5th-generation tensor cores (tcgen05 + TMEM) for head_dim 128 (sm_100a).
 //
-// Covers chatglm.cpp:655-717 for the sequences of a call that bring more than one token, in two launches for up to
-// kPrefillMaxSeq of them:
+// Covers chatglm.cpp:655-717 for the prompts of a call (n_past == 0, at least kPrefillMinTokens tokens), in two launches for up
+// to kPrefillMaxSeq of them:
 //   prefill_append_kernel  RoPE on k (:655-656) and the f16 append of the K rows and V^T columns (:668-675);
 //   prefill_attn_kernel    RoPE on q, q * 1/sqrt(d) (:686) and flash attention over the cache (:687-717).
 // An attention CTA works on TWO 128-row q tiles at a time that read the same K and V^T tiles: the same token rows of two
@@ -22,7 +22,7 @@
 // slower, because what the softmax warps issue delays the MMA warps, which need about a tenth of the issue slots.
 // O stays in tensor memory across KV tiles; a row's O is rescaled there only when its running maximum grows by more than
 // 2^8, otherwise the old reference maximum is kept (exact: the same reference enters numerator and denominator).
-// Masks (chatglm.cpp:689-707, at n_past == 0 only): causal (token t visible to row s iff t <= n_virtual + s; tiles right
+// Masks (chatglm.cpp:689-707): causal (token t visible to row s iff t <= n_virtual + s; tiles right
 // of the diagonal are skipped) or the ChatGLM-6B v1 prefix mask (every row but the last is blocked from the last token).
 // Tokens past the attended length: their scores are masked whatever the cache holds there, and the V^T tensor map of a
 // sequence ends at its attended length, so TMA fills the rest with zeros.
@@ -178,14 +178,13 @@ __device__ __forceinline__ void load_row8(Row8 &x, const PrefillSeq &ps, int rop
     // rope_table_kernel filled for this call, [stream][token].
     const int sc = min(s, sq.qlen - 1);
     if (rope_type == CGLM_ROPE_CHATGLM2) {           // dims [0, 64) as adjacent pairs: lanes 0..7, ladder steps 4 hl .. 4 hl + 3
-        const int row = ps.by_position ? sq.n_past + sc : sc;
-        const float4 *t = reinterpret_cast<const float4 *>(ps.angles + static_cast<long long>(row) * 32 + 4 * (hl & 7));
+        const float4 *t = reinterpret_cast<const float4 *>(ps.angles + static_cast<long long>(sc) * 32 + 4 * (hl & 7));
         x.a[0] = __ldg(t);
         x.a[1] = __ldg(t + 1);
     } else if (rope_type == CGLM_ROPE_CHATGLM) {     // each 64-dim half as pairs (i, i + 32): ladder steps 8 (hl & 3) .. + 7
         const bool second = hl >= 8;                 // by the position id, the second half by the block position id
-        const int p = sq.n_past + sc, lim = sq.n_ctx - 2;
-        const int row = ps.by_position ? (second ? max(p - lim, 0) : min(p, lim)) : (second ? sq.qlen + sc : sc);
+        const int lim = sq.n_ctx - 2;
+        const int row = ps.by_position ? (second ? max(sc - lim, 0) : min(sc, lim)) : (second ? sq.qlen + sc : sc);
         const float4 *t = reinterpret_cast<const float4 *>(ps.angles + static_cast<long long>(row) * 32 + 8 * (hl & 3));
 #pragma unroll
         for (int i = 0; i < 4; ++i) x.a[i] = __ldg(t + i);
@@ -394,7 +393,7 @@ __device__ __forceinline__ Unit unit_of(const PrefillTable &tab, const AttnShape
     }
     un.g = un.head[0] / sh.R;
     const int L = ps.sq.kv_before + ps.sq.qlen;
-    const int end = ps.causal ? min(L, ps.sq.kv_before + (un.tile[1] + 1) * kQTile) : L;   // one past the last visible token
+    const int end = sh.mask_type == CGLM_MASK_CAUSAL ? min(L, ps.sq.kv_before + (un.tile[1] + 1) * kQTile) : L;   // one past the last visible token
     un.n_step = (end + kStep - 1) / kStep;
     return un;
 }
@@ -642,6 +641,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
         const int row = 32 * gw + lane;           // TMEM lane
         const uint32_t lane_base = static_cast<uint32_t>(32 * gw) << 16;   // this warp's quarter of the TMEM lanes
         const uint32_t ts = tmem + 128 * w + lane_base, to = tmem + 256 + 128 * w + lane_base;
+        const bool causal = sh.mask_type == CGLM_MASK_CAUSAL;
         int t = 0;   // steps so far
         for (int k = 0, idx; w < n_groups && (idx = unit_index(k)) < n_units; ++k) {
             const Unit un = unit_of(tab, sh, idx);
@@ -651,7 +651,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
             float m_ref = -INFINITY, l_run = 0.f;   // reference maximum (log2 domain) and row sum relative to it
             // the last token a row may attend (inclusive); a row past S is computed like any other and not stored
             const int L = sq.kv_before + S, s_row = s0 + row;
-            const int row_last = ps.causal ? min(L - 1, sq.kv_before + s_row) : (ps.blocked && s_row < S - 1 ? L - 2 : L - 1);
+            const int row_last = causal ? min(L - 1, sq.kv_before + s_row) : (s_row < S - 1 ? L - 2 : L - 1);
             // One step: 64 tokens.  Masked and unmasked steps are separate code: in one loop the mask's selects are issued, if
             // predicated off, in every step.
             auto step = [&](int j, auto masked) {
@@ -735,7 +735,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
                 ++t;
             };
             // steps in which every row of this warp sees all 64 tokens
-            const int first_last = ps.causal ? min(L - 1, sq.kv_before + s0 + 32 * gw) : (ps.blocked ? L - 2 : L - 1);
+            const int first_last = causal ? min(L - 1, sq.kv_before + s0 + 32 * gw) : L - 2;
             const int n_clear = min(n_step, (first_last + 1) / kStep);
             int j = 0;
 #pragma unroll 1
@@ -822,8 +822,6 @@ cudaError_t launch_prefill(const LaunchCtx &cx, PrefillTable &tab, const CUtenso
         ps.block_begin = blocks;
         blocks += (S + kAppTokens - 1) / kAppTokens;
         tiles += static_cast<long long>(ps.n_q) * sh.H;
-        ps.causal = ps.sq.n_past == 0 && sh.mask_type == CGLM_MASK_CAUSAL;
-        ps.blocked = ps.sq.n_past == 0 && sh.mask_type == CGLM_MASK_CHATGLM;
         ps.vec = decode_rows_aligned(ps.sq.q, ps.sq.k, ps.sq.v, ps.sq.q_head_stride, ps.sq.kv_head_stride, nullptr, nullptr,
                                      (ps.sq.flags & CGLM_SEQ_QKV_F16) != 0) &&
                  ps.sq.q_tok_stride % 4 == 0 && ps.sq.kv_tok_stride % 4 == 0;
@@ -831,7 +829,7 @@ cudaError_t launch_prefill(const LaunchCtx &cx, PrefillTable &tab, const CUtenso
         // explicit position ids may not, so such a sequence gets a table of its own first.
         ps.angles = cx.rope_tab;
         ps.by_position = 1;
-        if (sh.rope_type != CGLM_ROPE_DISABLED && (ps.sq.position_ids || !cx.rope_tab || ps.sq.n_past + S > cx.rope_tab_len)) {
+        if (sh.rope_type != CGLM_ROPE_DISABLED && (ps.sq.position_ids || !cx.rope_tab || S > cx.rope_tab_len)) {
             const int n_entries = (sh.rope_type == CGLM_ROPE_CHATGLM ? 2 : 1) * S * 32;
             rope_table_kernel<<<(n_entries + 255) / 256, 256, 0, cx.stream>>>(sh, ps.sq, own_angles);
             ps.angles = own_angles;

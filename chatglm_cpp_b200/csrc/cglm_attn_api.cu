@@ -659,7 +659,7 @@ int forward_impl(cglm_kv_arena *a, const cglm_attn_seq *seqs, int n_seq, void *w
         if (!s.q || !s.k || !s.v || s.qlen <= 0 || s.n_past < 0 || s.slot < 0 || s.slot >= a->n_slots)
             return CGLM_ERR_INVALID_ARG;
         // qlen > 1 with n_past != 0 (a prompt fed in chunks) is served like the reference serves it: no mask at all
-        // (chatglm.cpp:689 masks only at n_past == 0), on the generic path
+        // (chatglm.cpp:689 masks only at n_past == 0), on the generic path (see kPrefillMinTokens)
         const bool partial = (s.flags & CGLM_SEQ_PARTIAL) != 0;
         if (partial ? !s.partial : !s.out) return CGLM_ERR_INVALID_ARG;
         // vector stores: out rows are written four elements at a time (16 bytes of f32, 8 of f16), partial rows 8 bytes
@@ -691,7 +691,7 @@ int forward_impl(cglm_kv_arena *a, const cglm_attn_seq *seqs, int n_seq, void *w
         if (is_fast[i]) {
             ++n_fast;
             decode_tiles += static_cast<long long>((L + kDecodeTile - 1) / kDecodeTile) * d.n_kv_head;
-        } else if (prefill_ok && s.qlen >= kPrefillMinTokens && (s.flags & ~(CGLM_SEQ_CACHE_SETTLED | CGLM_SEQ_QKV_F16 | CGLM_SEQ_OUT_F16)) == 0) {
+        } else if (prefill_ok && s.qlen >= kPrefillMinTokens && s.n_past == 0 && (s.flags & ~(CGLM_SEQ_CACHE_SETTLED | CGLM_SEQ_QKV_F16 | CGLM_SEQ_OUT_F16)) == 0) {
             is_fast[i] = 2;
             ++n_prefill;
             prefill_bytes += prefill_angle_bytes(s.qlen);

@@ -371,8 +371,8 @@ inline bool decode_rows_aligned(const float *q, const float *k, const float *v, 
     const uintptr_t out_bits = reinterpret_cast<uintptr_t>(q_roped) | reinterpret_cast<uintptr_t>(k_roped);
     return (in_bits & (qkv_f16 ? 7 : 15)) == 0 && (out_bits & 15) == 0 && q_head_stride % 4 == 0 && kv_head_stride % 4 == 0;
 }
-// tcgen05 path of sequences with more than one token (head_dim 128): what the two launches know about up to kPrefillMaxSeq of
-// them, passed by value.  A sequence's V^T tensor map ends at its attended length.
+// tcgen05 path of prompts (n_past == 0, head_dim 128): what the two launches know about up to kPrefillMaxSeq of them, passed by
+// value.  A sequence's V^T tensor map ends at its attended length.
 constexpr int kPrefillMaxSeq = 8;
 constexpr int kPrefillMaxCtas = 148;   // x 64 KiB of q tiles: what the Linear kernels' scratch holds
 enum { kPrefillSingle = 0, kPrefillPairHeads = 1, kPrefillPairTiles = 2 };   // q tiles per CTA, and which two
@@ -381,7 +381,6 @@ struct PrefillSeq {
     const float2 *angles;   // arena's table (by_position) or this call's [stream][token][32]
     int by_position;
     int vec;                // q, k, v rows can be read four elements at a time
-    int causal, blocked;    // mask at n_past == 0: causal, or the v1 prefix mask
     int n_q;                // 128-row tiles
     int block_begin;        // first 64-token block of the append kernel
     int unit_begin;         // first CTA of the attention kernel
@@ -393,8 +392,13 @@ struct PrefillTable {
 };
 size_t prefill_angle_bytes(int S);
 cudaError_t launch_prefill(const LaunchCtx &cx, PrefillTable &tab, const CUtensorMap &k_map, float2 *own_angles);
-// Shorter ones run on the generic path.
-constexpr int kPrefillMinTokens = 2;
+// Shorter prompts, and every chunk at n_past > 0, multiply f32 q and f32 probabilities with the cache on the generic path: in
+// float64 terms 2.4e-7 relative for 57 tokens and 1.3e-6 for 512 tokens behind 4096, where the f16 operands of the tensor cores
+// give 1.9e-4 and 3.0e-4.  The f32 route is the slower one by far (57 tokens 71 us against 9, 127 tokens 229 against 11, 512
+// behind 4096 52 ms against 63 us).  Splitting both operands into two f16 terms is not enough to go back: sums that stay in
+// tensor memory are truncated at every MMA (2.8e-6 relative after 512 products of one sign, 2.6e-5 after 4096, against
+// 1e-6 for sequential f32 sums), so the sums of more than a few steps have to be kept outside.
+constexpr int kPrefillMinTokens = 128;
 // fused query_key_value Linear + RoPE + append for one-token sequences (tcgen05): x_map f16 {64, n_tok, K/64} box
 // {64, qkv_linear_x_rows(n_tok), kb}, w_map f16 {64, n_feat, K/64} box {64, 32, kb}, both 128-byte swizzled;
 // kb (64-k blocks per box) <= qkv_linear_k_blocks(n_tok, K)
