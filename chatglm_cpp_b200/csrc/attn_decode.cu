@@ -1340,20 +1340,26 @@ int decode_max_ctas(int n_sm) { return 2 * n_sm; }   // bound used to size scrat
 
 // Thread blocks per cluster with which decode_cluster_kernel takes a launch, 0: the persistent kernel takes it.
 // Clusters of eight up to 8 items (sequences x kv heads), of four up to a quarter of the SMs, of two up to half of them: one
-// thread block per SM with room for the clusters' placement (16 clusters of eight do not fit the 148 SMs at once: 14.4 us per
-// launch against 7.4 for 8).  The line is the longest item, because an item cannot borrow another's warps: 8 tiles (512
-// tokens) per thread block.  Measured, us per launch in a chain, f16 activations, persistent kernel -> clusters:
+// thread block per SM, and only as many clusters as the device runs at once.  A cluster lies inside one group of SMs, so
+// that is fewer than n_sm / n_cta (on a B200 15 of eight, 33 of four, 74 of two), and one cluster more is a second wave: 34 to
+// 36 items of 200 tokens 14.0 us per launch with clusters of four, 9.9 with the persistent kernel, 6.7 with clusters of two.
+// The line is the longest item, because an item cannot borrow another's warps: 8 tiles (512 tokens) per thread block.  Where
+// the items divide the SMs evenly the persistent kernel's spans end where (equal) items do, which is its best case, and the line
+// is 4 tiles (74 items: 512 tokens 14.7 us against 16.3 with clusters of two, 400 tokens 12.9 against 12.4).  Measured, us per launch in a chain, f16 activations, persistent kernel -> clusters:
 //   8 thread blocks, 1 / 4 sequences   512 tokens 10.5 -> 6.7 / 10.9 -> 7.4   2048 13.5 -> 10.1 / 20.3 -> 12.4   4096 17.6 -> 16.6 / 35.7 -> 19.0
 //   4 thread blocks, 16 sequences      512 tokens 22.9 -> 10.0   1024 25.2 -> 13.7   2048 28.5 -> 20.5   4096 27.1 -> 28.2
 //   2 thread blocks, 32 sequences      512 tokens 21.5 -> 13.6   1024 25.2 -> 20.4   2048 27.4 -> 28.4
 //   one q head per kv head, 32 of them: 2048 tokens 20.2 -> 19.3 with 4, two sequences 1024 tokens 21.3 -> 19.1 with 2
-int decode_cluster_ctas(const DecodeTable &tab, int G, int n_sm) {
+int decode_cluster_ctas(const DecodeTable &tab, int G, int n_sm, int device) {
     const int n_items = tab.n_seq * G;
     if (tab.n_seq > kDecodeClusterMaxSeq || 2 * n_items > n_sm) return 0;
-    const int n_cta = n_items <= 8 ? 8 : (4 * n_items <= n_sm ? 4 : 2);
     int longest = 0;
     for (int i = 0; i < tab.n_seq; ++i) longest = std::max(longest, tab.prefix[i + 1] - tab.prefix[i]);
-    return longest <= 8 * n_cta ? n_cta : 0;
+    int n_cta = n_items <= 8 ? 8 : (4 * n_items <= n_sm ? 4 : 2);
+    while (n_cta > 1 && n_items > decode_cluster_resident(device, n_cta)) n_cta /= 2;
+    if (n_cta < 2) return 0;
+    const int line = n_items > 8 && n_sm % n_items == 0 ? 4 : 8;
+    return longest <= line * n_cta ? n_cta : 0;
 }
 
 cudaError_t launch_decode(const LaunchCtx &cx, const DecodeTableDyn &tab, bool n_past_on_device, const XchgDev *xchg) {
@@ -1363,7 +1369,7 @@ cudaError_t launch_decode(const LaunchCtx &cx, const DecodeTableDyn &tab, bool n
         return cudaSuccess;
     }
     if (!xchg) {
-        const int n_cta = decode_cluster_ctas(tab, cx.shape.G, cx.n_sm);
+        const int n_cta = decode_cluster_ctas(tab, cx.shape.G, cx.n_sm, cx.device);
         if (n_cta > 0) return launch_decode_cluster(cx, tab, n_cta);
     }
     static PerDeviceOnce configured;

@@ -419,15 +419,20 @@ decode_cluster_kernel(const __grid_constant__ ClusterTable<kCap> tab, AttnShape 
 }
 
 template <int kCta, int kCap>
+cudaError_t configure(int device) {
+    static PerDeviceOnce configured;
+    if (!configured.needed(device)) return cudaSuccess;
+    cudaError_t e = require_current_device(device);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_cluster_kernel<kCta, kCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e == cudaSuccess) configured.mark(device);
+    return e;
+}
+
+template <int kCta, int kCap>
 cudaError_t launch(const LaunchCtx &cx, const DecodeTable &tab) {
     static thread_local ClusterTable<kCap> t;
-    static PerDeviceOnce configured;
-    if (configured.needed(cx.device)) {
-        cudaError_t e = require_current_device(cx.device);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_cluster_kernel<kCta, kCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        if (e != cudaSuccess) return e;
-        configured.mark(cx.device);
-    }
+    cudaError_t e = configure<kCta, kCap>(cx.device);
+    if (e != cudaSuccess) return e;
     t.n_seq = tab.n_seq;
     for (int i = 0; i < 2; ++i) { t.gate[i] = tab.gate[i]; t.gate_value[i] = tab.gate_value[i]; }
     for (int i = 0; i < tab.n_seq; ++i) t.seqs[i] = tab.seqs[i];
@@ -443,13 +448,39 @@ cudaError_t launch(const LaunchCtx &cx, const DecodeTable &tab) {
     cfg.stream = cx.stream;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, decode_cluster_kernel<kCta, kCap>, t, cx.shape, cx.k_base, cx.v_base, cx.hdr, cx.rope_tab,
+    e = cudaLaunchKernelEx(&cfg, decode_cluster_kernel<kCta, kCap>, t, cx.shape, cx.k_base, cx.v_base, cx.hdr, cx.rope_tab,
                                        cx.rope_tab_len);
     g_launch_count += 1;
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+template <int kCta>
+int resident(int device) {
+    static std::atomic<int> known[kMaxDevices];   // 1 + the count, 0: not asked yet
+    const bool keep = device >= 0 && device < kMaxDevices;
+    const int k = keep ? known[device].load(std::memory_order_relaxed) : 0;
+    if (k > 0) return k - 1;
+    if (configure<kCta, 8>(device) != cudaSuccess) return 0;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kCta; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kCta);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, decode_cluster_kernel<kCta, 8>, &cfg) != cudaSuccess) return 0;
+    if (keep) known[device].store(n + 1, std::memory_order_relaxed);
+    return n;
+}
+
 }  // namespace
+
+int decode_cluster_resident(int device, int n_cta) {
+    return n_cta == 8 ? resident<8>(device) : (n_cta == 4 ? resident<4>(device) : resident<2>(device));
+}
 
 cudaError_t launch_decode_cluster(const LaunchCtx &cx, const DecodeTable &tab, int n_cta) {
     static_assert(kDecodeClusterMaxSeq == 64, "the larger table");

@@ -363,6 +363,8 @@ cudaError_t launch_decode(const LaunchCtx &cx, const DecodeTableDyn &tab, bool n
 // the same for a small launch, one cluster of n_cta (2, 4, 8) thread blocks per (sequence, kv head)
 constexpr int kDecodeClusterMaxSeq = 64;
 cudaError_t launch_decode_cluster(const LaunchCtx &cx, const DecodeTable &tab, int n_cta);
+// how many clusters of n_cta such thread blocks the (current) device runs at once; 0 when that cannot be told
+int decode_cluster_resident(int device, int n_cta);
 // The decode kernel reads q/k/v head rows four elements at a time (sixteen bytes of f32, eight of f16) and writes the
 // optional roped copies sixteen bytes at a time.
 inline bool decode_rows_aligned(const float *q, const float *k, const float *v, long long q_head_stride,

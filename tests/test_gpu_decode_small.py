@@ -24,6 +24,10 @@ LENS8 = [0, 1, 30, 31, 32, 127, 128, 129]
     (6, 2, O.ROPE_DISABLED, O.MASK_CAUSAL, 0, 520, LENS8),                                # three q heads per kv head
     (32, 32, O.ROPE_CHATGLM, O.MASK_CHATGLM, 0, 1096, [700, 1023]),                       # clusters of two, one q head each
     (4, 4, O.ROPE_CHATGLM, O.MASK_CHATGLM, 5, 520, LENS8),                                # a P-Tuning prefix
+    (4, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 264, [7 * i % 256 for i in range(16)]),     # 32 items: clusters of four
+    (4, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 264, [7 * i % 256 for i in range(18)]),     # 36: more than are resident
+    (4, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 584, [512] * 37),                           # 74, two per SM: past its line
+    (4, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL, 0, 584, [511] * 37),                           # and on it
 ])
 @pytest.mark.parametrize("on_device", [False, True])
 def test_small_decode(H, G, rope, mask, V, M, lens, on_device):
