@@ -50,6 +50,9 @@ constexpr int kStages = 5;                    // ring of K and V^T tiles: K(0), 
 constexpr int kTmemCols = 512;                // group w: S at columns 128 w, P buffers at 128 w + 64 and + 96, O at 256 + 128 w
 constexpr float kRescaleThreshold = 8.f;      // log2 units a row's maximum may grow before O is rescaled
 constexpr float kLog2e = 1.4426950408889634f;
+// Reference maximum of a row that has seen no score above -inf (masked tokens, keys that overflowed f16): its exponents are
+// ex2(-inf - this) = 0, not NaN.
+constexpr float kNoMax = -1.0e30f;
 
 // instruction descriptors of tcgen05.mma.kind::f16: D = f32, A = B = f16, both K-major, M = 128, N = 64 (scores) / 128 (P V)
 constexpr uint32_t kIdescS = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
@@ -648,7 +651,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
             const PrefillSeq &ps = tab.seqs[un.seq];
             const SeqDev &sq = ps.sq;
             const int S = sq.qlen, h = w ? un.head[1] : un.head[0], s0 = (w ? un.tile[1] : un.tile[0]) * kQTile, n_step = un.n_step;
-            float m_ref = -INFINITY, l_run = 0.f;   // reference maximum (log2 domain) and row sum relative to it
+            float m_ref = kNoMax, l_run = 0.f;   // reference maximum (log2 domain) and row sum relative to it
             // the last token a row may attend (inclusive); a row past S is computed like any other and not stored
             const int L = sq.kv_before + S, s_row = s0 + row;
             const int row_last = causal ? min(L - 1, sq.kv_before + s_row) : (s_row < S - 1 ? L - 2 : L - 1);
@@ -682,10 +685,10 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
                 for (int i = 4; i < kStep / 2; ++i) mx4[i & 3] = max3(mx4[i & 3], sv[i].x, sv[i].y);
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * kLog2e;
                 // keep the old reference unless the maximum outgrew it by more than the threshold
-                const bool grow = mx > m_ref + kRescaleThreshold;   // also true for the first visible step (m_ref = -inf)
+                const bool grow = mx > m_ref + kRescaleThreshold;   // also true for the first step with a score above -inf
                 if (__any_sync(0xffffffffu, grow)) {
                     const float m_new = grow ? mx : m_ref;
-                    const float alpha = grow ? ex2_approx(m_ref - m_new) : 1.f;   // 0 when m_ref was -inf
+                    const float alpha = grow ? ex2_approx(m_ref - m_new) : 1.f;   // 0 when m_ref was kNoMax
                     l_run *= alpha;
                     m_ref = m_new;
                     if (j > 0) {
@@ -709,8 +712,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
                         }
                     }
                 }
-                const float m_base = decltype(masked)::value && m_ref == -INFINITY ? 0.f : m_ref;   // a row that has seen nothing yet: every p is 0
-                const float2 lg = make_float2(kLog2e, kLog2e), mb = make_float2(-m_base, -m_base);
+                const float2 lg = make_float2(kLog2e, kLog2e), mb = make_float2(-m_ref, -m_ref);
                 float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
                 for (int ch = 0; ch < kStep / 32; ++ch) {

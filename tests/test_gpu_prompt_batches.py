@@ -119,3 +119,29 @@ def test_short_prompts_and_chunks_keep_f32_operands(H, G, rope, mask, V, chunks,
         rel = float((torch.from_numpy(got).double() - exact).norm() / exact.norm())
         assert rel <= 8 * 2.0 ** -24 * (128 + T) ** 0.5, (P, S, rel)
     arena.close()
+
+
+@pytest.mark.parametrize("H,G,S", [(6, 2, 300), (32, 2, 600), (5, 5, 400)])   # one q tile per CTA; two heads, two row tiles
+def test_prompt_rows_whose_first_scores_are_minus_infinity(H, G, S):
+    """Keys of the first 150 tokens overflow f16 (to -inf in a dimension that RoPE leaves alone, where every q is positive): their
+    scores are -inf and their weights 0.  Rows from 150 on attend the tokens behind them; the reference is float64 over those."""
+    from chatglm_cpp_b200 import _lib
+    from chatglm_cpp_b200 import attention as A
+    N, R = 150, H // G
+    desc = make_desc(H, G, 128, 640)
+    rng = np.random.default_rng(S)
+    arena, ws = A.KVArena(desc, 1), A.Workspace(desc, 1, S)
+    x = rng.standard_normal((S, qkv_width(desc, False))).astype(np.float32)
+    x[:, 127:H * 128:128] = np.abs(x[:, 127:H * 128:128]) + 0.1
+    x[:N, H * 128 + 127:(H + G) * 128:128] = -1e6
+    before = _lib.lib().cglm_launch_count()
+    out, qr, _ = A.BasicAttention(arena, 0, ws).forward(torch.from_numpy(x).cuda(), 0, want_roped=True)
+    torch.cuda.synchronize()
+    assert ws.status() == 0 and _lib.lib().cglm_launch_count() - before == 2
+    k, v = arena.k_cache(0)[:, N:S].double().cpu(), arena.v_cache(0)[:, :, N:S].double().cpu()
+    assert torch.isneginf(arena.k_cache(0)[:, :N, 127]).all()
+    sc = torch.einsum("sgrd,gtd->sgrt", qr[N:].double().cpu().view(S - N, G, R, 128), k) / 128 ** 0.5
+    sc.masked_fill_((torch.arange(S - N)[None] > torch.arange(S - N)[:, None])[:, None, None], float("-inf"))
+    want = torch.einsum("sgrt,gdt->sgrd", torch.softmax(sc, -1), v).reshape(S - N, H * 128)
+    assert_out_close(out[N:].cpu().numpy(), want.numpy().astype(np.float32), f"{S} tokens")
+    arena.close()
