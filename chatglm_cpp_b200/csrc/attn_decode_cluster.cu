@@ -35,7 +35,7 @@ constexpr int kSmemBytes = 117248;
 constexpr int kRoundsAhead = 4;       // rounds of the cluster asked for in L2 before the wait
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
-// Reference point of the exponents where everything seen so far is masked (maximum -inf): ex2(-inf - this) is 0, not NaN.
+// Running maximum before the first score above -inf (none seen, or keys that overflowed f16): ex2(-inf - this) is 0, not NaN.
 constexpr float kNoMax = -1.0e30f;
 
 template <int kCap>
@@ -226,7 +226,7 @@ decode_cluster_kernel(const __grid_constant__ ClusterTable<kCap> tab, AttnShape 
     float o[16][4];
 #pragma unroll
     for (int i = 0; i < 16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // rows r8 and r8 + 8; this lane's share of the sums
+    float m_run[2] = {kNoMax, kNoMax}, l_run[2] = {0.f, 0.f};   // rows r8 and r8 + 8; this lane's share of the sums
     const __half *const qa = &sm.q[r8][8 * c], *const qb = &sm.q[r8 + 8][8 * c];
 #pragma unroll 1
     for (; tok0 < L; tok0 += tok_step) {
@@ -331,7 +331,7 @@ decode_cluster_kernel(const __grid_constant__ ClusterTable<kCap> tab, AttnShape 
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int r = r8 + 8 * h;
-            const float m_star = fmaxf(fmaxf(fmaxf(sm.stats[0][r], sm.stats[1][r]), fmaxf(sm.stats[2][r], sm.stats[3][r])), kNoMax);
+            const float m_star = fmaxf(fmaxf(sm.stats[0][r], sm.stats[1][r]), fmaxf(sm.stats[2][r], sm.stats[3][r]));
             a[h] = ex2_approx(m_run[h] - m_star);
         }
         // float2 unit u of row r lives at unit u ^ 4(r & 3): conflict-free stores here, and 16-byte reads below
@@ -348,7 +348,7 @@ decode_cluster_kernel(const __grid_constant__ ClusterTable<kCap> tab, AttnShape 
     if (tid < kRows) {
         m_cta = fmaxf(fmaxf(sm.stats[0][tid], sm.stats[1][tid]), fmaxf(sm.stats[2][tid], sm.stats[3][tid]));
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) l_cta += sm.stats[w][kRows + tid] * ex2_approx(sm.stats[w][tid] - fmaxf(m_cta, kNoMax));
+        for (int w = 0; w < kWarps; ++w) l_cta += sm.stats[w][kRows + tid] * ex2_approx(sm.stats[w][tid] - m_cta);
     }
     __syncthreads();
     if (tid < kRows) {

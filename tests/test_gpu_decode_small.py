@@ -54,6 +54,30 @@ def test_stale_cache_rows_behind_the_appended_token_do_not_reach_the_result():
         arena.close()
 
 
+@pytest.mark.parametrize("G,P", [(1, 500), (2, 2047), (16, 700), (32, 300)])   # clusters of eight (twice), four, two
+@pytest.mark.parametrize("lo,hi", [(0, 64), (96, 300)])
+def test_tokens_whose_scores_are_minus_infinity(G, P, lo, hi):
+    """Cached keys of tokens [lo, hi) are -inf in a dimension where every q is positive: the scores are -inf and the weights 0, also
+    where everything that a warp sees at first is such a token.  The reference is float64 over the other tokens."""
+    from chatglm_cpp_b200 import attention as A
+    desc = make_desc(2 * G, G, 128, 2056)
+    rng = np.random.default_rng(G + lo)
+    arena, ws = A.KVArena(desc, 1), A.Workspace(desc, 1, 1)
+    k, v = random_cache(rng, desc, P)
+    k[:, lo:hi, 127] = 0xFC00
+    upload_cache(arena, 0, k, v)
+    x = rng.standard_normal((1, qkv_width(desc, False))).astype(np.float32)
+    x[:, 127:2 * G * 128:128] = np.abs(x[:, 127:2 * G * 128:128]) + 0.1
+    out, qr, _ = A.BasicAttention(arena, 0, ws).forward(torch.from_numpy(x).cuda(), P, want_roped=True)
+    torch.cuda.synchronize()
+    assert ws.status() == 0
+    keep = [t for t in range(P + 1) if not lo <= t < hi]
+    kk, vv = arena.k_cache(0)[:, keep].double().cpu(), arena.v_cache(0)[:, :, keep].double().cpu()
+    w = torch.softmax(torch.einsum("grd,gtd->grt", qr.double().cpu().view(G, 2, 128), kk) / 128 ** 0.5, -1)
+    assert_out_close(out.cpu().numpy(), torch.einsum("grt,gdt->grd", w, vv).reshape(1, -1).numpy().astype(np.float32), f"{G} kv heads")
+    arena.close()
+
+
 @pytest.mark.parametrize("G", [8, 10, 13, 16, 20])
 def test_merge_of_items_cut_into_many_parts(G):
     """One sequence just past the clusters' line, cut over one thread block per SM: 7 to 18 parts per item, i.e. fewer than one
