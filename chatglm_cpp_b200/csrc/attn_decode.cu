@@ -602,7 +602,9 @@ __device__ __forceinline__ void merge_staged(const DeliverArgs *da, const Global
     float *const slots = da->slots;
     uint64_t *const bars = da->bars;
     if (t == 0) {
-        fence_proxy_async();   // the parts are other threads' plain stores, acquired with the count
+        // The parts are plain stores to global memory, by other thread blocks and (group partials) by this one, which the count
+        // ordered before this thread: the fence carries that order to the bulk copies, which are of the async proxy.
+        fence_proxy_async_global();
         mbar_arrive_expect_tx(&bars[0], static_cast<uint32_t>(n_first) * kBytes);
         if (n > n_first) mbar_arrive_expect_tx(&bars[1], static_cast<uint32_t>(n - n_first) * kBytes);
 #pragma unroll 1
@@ -825,7 +827,8 @@ __device__ __noinline__ void deliver_part(const DeliverArgs *da, long long b, in
         __threadfence();
         merge(mc.partials, b0, first_cta_slot, gb0, gb1,
               mc.gpartials + (grp * 2 + group_slot(grp, b0)) * kDecodePartialFloats, 0);
-        __threadfence();   // every member publishes its piece of the group partial before the leader counts the group
+        __threadfence();   // every member publishes its piece of the group partial before the leader counts the group,
+        fence_proxy_async();   // and has read the ring before the second level's copies write it
         if (!lead(mc.counters + item, static_cast<int>(g1 - g0 + 1))) return;
         base = mc.gpartials; k_first = g0; first_slot = first_grp_slot; k0 = g0; k1 = g1;
     }

@@ -85,6 +85,28 @@ def test_merge_of_items_cut_into_many_parts(G):
     run_decode_batch(make_desc(2 * G, G, 128, 4168, 0, O.ROPE_CHATGLM2, 10000.0, O.MASK_CAUSAL), [4150], seed=G)
 
 
+@pytest.mark.parametrize("G,P", [(8, 4150), (13, 4150), (2, 20000)])   # one and two rounds of copies, two levels of merging
+def test_merged_parts_are_those_of_the_launch(G, P):
+    """Launches with two inputs in turn through the same scratch: every result has the bits of the first launch with that input, so
+    no part, group partial or slot of the tile ring is one that an earlier launch left behind."""
+    from chatglm_cpp_b200 import attention as A
+    desc = make_desc(2 * G, G, 128, P + 72)
+    rng = np.random.default_rng(G)
+    arena, ws = A.KVArena(desc, 2), A.Workspace(desc, 1, 1)
+    attn, x = [], []
+    for slot in range(2):
+        k, v = random_cache(rng, desc, P)
+        upload_cache(arena, slot, k, v)
+        attn.append(A.BasicAttention(arena, slot, ws))
+        x.append(torch.from_numpy(rng.standard_normal((1, qkv_width(desc, False))).astype(np.float32)).cuda())
+    first = [attn[i].forward(x[i], P) for i in range(2)]
+    outs = [attn[i % 2].forward(x[i % 2], P) for i in range(300)]
+    torch.cuda.synchronize()
+    assert ws.status() == 0 and not torch.equal(first[0], first[1])
+    assert all(torch.equal(o, first[i % 2]) for i, o in enumerate(outs))
+    arena.close()
+
+
 @pytest.mark.parametrize("n_tok,n_in,n_out", [(128, 256, 128), (128, 512, 4096), (33, 4096, 4608), (1, 128, 128), (17, 4160, 256)])
 def test_linear_k_split_over_a_cluster(n_tok, n_in, n_out):
     """Fewer weight blocks than the sums need room, one block per thread block, token counts that no CTA's share divides, a k that
