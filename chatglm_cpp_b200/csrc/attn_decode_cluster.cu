@@ -364,17 +364,20 @@ decode_cluster_kernel(const __grid_constant__ ClusterTable<kCap> tab, AttnShape 
     }
     cluster_sync();
 
-    // ---- the thread blocks of the cluster: rank k finishes dims [128 k / kCta, 128 (k + 1) / kCta) of all rows -------------
-    {
+    // ---- the thread blocks of the cluster: rank k finishes dims [128 k / kCta, 128 (k + 1) / kCta) of the rows -------------
+    // Only values that reach a store below are read from the peers: what keeps a peer's shared memory alive past these reads is
+    // that the stores, and so the values, come before this thread's last arrival.
+    if ((tid >> 3) < R && L > 0 && !sm.abort_flag) {
         constexpr int kUnits = kRows / kCta / 2 > 0 ? kRows / kCta / 2 : 1;   // float2 units per thread, eight threads per row
         const int r = tid >> 3, u0 = rank * (kD / 2 / kCta) + (tid & 7) * kUnits;
         const float *stat = &sm.stats[0][r];
+        const bool want_l = !(flags & CGLM_SEQ_PARTIAL) || (rank == 0 && (tid & 7) == 0);
         float m[kCta], l[kCta];
         float2 v[kCta][kUnits];
 #pragma unroll
         for (int k = 0; k < kCta; ++k) {
             m[k] = ld_peer(peer_addr(stat, k));
-            l[k] = ld_peer(peer_addr(stat + kRows, k));
+            l[k] = want_l ? ld_peer(peer_addr(stat + kRows, k)) : 0.f;
 #pragma unroll
             for (int i = 0; i < kUnits; ++i) v[k][i] = ld_peer2(peer_addr(&sm.part[0][r * kD + 2 * ((u0 + i) ^ (4 * (r & 3)))], k));
         }
@@ -391,29 +394,26 @@ decode_cluster_kernel(const __grid_constant__ ClusterTable<kCap> tab, AttnShape 
 #pragma unroll
             for (int i = 0; i < kUnits; ++i) { acc[i].x += w * v[k][i].x; acc[i].y += w * v[k][i].y; }
         }
-        if (r < R && L > 0 && !sm.abort_flag) {
-            const int head = g * R + r;
-            if (flags & CGLM_SEQ_PARTIAL) {
-                float *po = sm.sq.partial + static_cast<long long>(head) * (kD + 2);
+        const int head = g * R + r;
+        if (flags & CGLM_SEQ_PARTIAL) {
+            float *po = sm.sq.partial + static_cast<long long>(head) * (kD + 2);
 #pragma unroll
-                for (int i = 0; i < kUnits; ++i) *reinterpret_cast<float2 *>(po + 2 * (u0 + i)) = acc[i];
-                if (rank == 0 && (tid & 7) == 0) { po[kD] = m_star * kLn2; po[kD + 1] = den; }
-            } else {
-                const float inv = 1.f / den;
+            for (int i = 0; i < kUnits; ++i) *reinterpret_cast<float2 *>(po + 2 * (u0 + i)) = acc[i];
+            if (rank == 0 && (tid & 7) == 0) { po[kD] = m_star * kLn2; po[kD + 1] = den; }
+        } else {
+            const float inv = 1.f / den;
 #pragma unroll
-                for (int i = 0; i < kUnits; ++i) {
-                    const long long e = static_cast<long long>(head) * kD + 2 * (u0 + i);
-                    if (flags & CGLM_SEQ_OUT_F16) {
-                        *reinterpret_cast<uint32_t *>(reinterpret_cast<__half *>(sm.sq.out) + e) = pack_half2(acc[i].x * inv, acc[i].y * inv);
-                    } else {
-                        *reinterpret_cast<float2 *>(sm.sq.out + e) = make_float2(acc[i].x * inv, acc[i].y * inv);
-                    }
+            for (int i = 0; i < kUnits; ++i) {
+                const long long e = static_cast<long long>(head) * kD + 2 * (u0 + i);
+                if (flags & CGLM_SEQ_OUT_F16) {
+                    *reinterpret_cast<uint32_t *>(reinterpret_cast<__half *>(sm.sq.out) + e) = pack_half2(acc[i].x * inv, acc[i].y * inv);
+                } else {
+                    *reinterpret_cast<float2 *>(sm.sq.out + e) = make_float2(acc[i].x * inv, acc[i].y * inv);
                 }
             }
         }
     }
-    // A thread block's shared memory outlives its peers' reads, whose values are in registers by now: nothing to order, and
-    // the output stores are not waited for.
+    // Nothing to order, and the output stores are not waited for.
     __syncwarp();
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }

@@ -78,6 +78,36 @@ def test_tokens_whose_scores_are_minus_infinity(G, P, lo, hi):
     arena.close()
 
 
+@pytest.mark.parametrize("R", [1, 2, 3, 15, 16])
+@pytest.mark.parametrize("G", [2, 16, 32])   # clusters of eight, four and two
+def test_rows_of_an_item_in_launches_back_to_back(R, G):
+    """Items of fewer q heads than the sixteen rows that an MMA has, whole and as un-normalised partials, 100 launches each with
+    nothing in between: every one gives the bits of the first, which the oracle holds."""
+    from chatglm_cpp_b200 import _lib
+    from chatglm_cpp_b200 import attention as A
+    H, P = R * G, 190
+    desc = make_desc(H, G, 128, 264)
+    rng = np.random.default_rng(H)
+    arena, ws = A.KVArena(desc, 1), A.Workspace(desc, 1, 1)
+    k, v = random_cache(rng, desc, P)
+    upload_cache(arena, 0, k, v)
+    x = rng.standard_normal((1, qkv_width(desc, False))).astype(np.float32)
+    qkv = torch.from_numpy(x).cuda()
+    attn = A.BasicAttention(arena, 0, ws)
+    outs = [attn.forward(qkv, P) for _ in range(100)]
+    parts = [torch.zeros(H, 130, device="cuda") for _ in range(100)]
+    for p in parts:
+        A.forward_batch(arena, ws, [A.SeqCall(qkv=qkv, slot=0, n_past=P, n_ctx=0, partial=p, flags=_lib.SEQ_PARTIAL)], False)
+    torch.cuda.synchronize()
+    assert ws.status() == 0
+    assert all(torch.equal(o, outs[0]) for o in outs) and all(torch.equal(p, parts[0]) for p in parts)
+    want = O.attn_forward(oracle_cfg(desc, "f32"), x, False, k, v, P)
+    assert_out_close(outs[0].cpu().numpy(), want, f"{H} q heads, {G} kv heads")
+    whole = (parts[0][:, :128] / parts[0][:, 129:]).reshape(1, -1)
+    assert_out_close(whole.cpu().numpy(), want, "partial")
+    arena.close()
+
+
 @pytest.mark.parametrize("G", [8, 10, 13, 16, 20])
 def test_merge_of_items_cut_into_many_parts(G):
     """One sequence just past the clusters' line, cut over one thread block per SM: 7 to 18 parts per item, i.e. fewer than one
