@@ -116,7 +116,9 @@ __device__ __forceinline__ bool mbar_try_wait_for(uint64_t *bar, uint32_t parity
 // on without touching the barrier again.  *abort_flag lives in shared memory.  A waiting warp suspends in the barrier instead
 // of polling (polls take issue slots from the warps that work), so the wait is bounded by time: at most kWaitLimitNs.
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+// started: for a wait that may begin before this grid's dependency wait, a word that is set once the kernel in front has
+// completed; the time until then does not count.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort_flag, volatile int *started = nullptr) {
     if (mbar_try_wait(bar, parity)) {   // nothing else on the path of a wait that is already met
         return true;
     }
@@ -130,7 +132,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
         }
         unsigned long long now;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-        if (t0 == 0) t0 = now;
+        if (t0 == 0 || (started && !*started)) {
+            t0 = now;
+            i = 0;
+        }
         if (now - t0 > kWaitLimitNs) break;
     }
     *abort_flag = 1;

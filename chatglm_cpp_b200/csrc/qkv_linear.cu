@@ -66,6 +66,7 @@ struct __align__(1024) QkvSmem {
     uint64_t acc_full;
     uint32_t tmem_base;
     int abort_flag;
+    int started;             // the TMA warp has passed the dependency wait: x is on its way
     // 1024-byte aligned: n_stages stages of (kb x tiles of x_rows rows | kb W tiles), then read_over_slack(): the MMA
     // reads 128 rows from every x tile, whatever x_rows is
     __align__(1024) uint8_t ring[1];
@@ -122,7 +123,7 @@ qkv_linear_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     const int k_first = static_cast<int>(blockIdx.x) % n_k;
 
     if (tid == 0) {
-        sm.abort_flag = 0;
+        sm.abort_flag = sm.started = 0;
         for (int s = 0; s < n_stages; ++s) {
             mbar_init(&sm.full[s], 1);
             mbar_init(&sm.empty[s], 1);
@@ -153,6 +154,7 @@ qkv_linear_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
                 tma_load_3d(sm.ring + i * stage_bytes + x_bytes, &w_map, 0, f0, ((i + k_first) % n_k) * kb, &sm.full[i]);
             }
             asm volatile("griddepcontrol.wait;" ::: "memory");
+            *static_cast<volatile int *>(&sm.started) = 1;
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             // rows of x past n_tok are outside the tensor map and arrive as zeros: the box is x_rows tokens
             for (int i = 0; i < pre; ++i) tma_load_3d(sm.ring + i * stage_bytes, &x_map, 0, tok0, ((i + k_first) % n_k) * kb, &sm.full[i]);
@@ -169,7 +171,7 @@ qkv_linear_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     } else if (warp == kMmaWarp) {
         if (lane == 0) {
             for (int i = 0, st = 0, round = 0; i < n_k; ++i) {
-                if (!mbar_wait_bounded(&sm.full[st], round & 1u, &sm.abort_flag)) break;
+                if (!mbar_wait_bounded(&sm.full[st], round & 1u, &sm.abort_flag, &sm.started)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t xs = smem_u32(sm.ring + st * stage_bytes), wsm = xs + x_bytes;
 #pragma unroll 1
@@ -325,6 +327,7 @@ struct __align__(1024) FmSmem {
     uint64_t acc_full;
     uint32_t tmem_base;
     int abort_flag;
+    int started;             // the TMA warp has passed the dependency wait: x is on its way
     // 1024-byte aligned: n_stages stages of (kb x tiles of n_box token rows | kb W tiles); after the last MMA this CTA's
     // sums [token][128]
     __align__(1024) uint8_t ring[1];
@@ -472,7 +475,7 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     const int stage_bytes = x_bytes + kb * kFmWBytes;
 
     if (tid == 0) {
-        sm.abort_flag = 0;
+        sm.abort_flag = sm.started = 0;
         for (int s = 0; s < n_stages; ++s) {
             mbar_init(&sm.full[s], 1);
             mbar_init(&sm.empty[s], 1);
@@ -499,6 +502,7 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
                 tma_load_3d(sm.ring + i * stage_bytes + x_bytes, &w_map, 0, f0, k_base + i * kb, &sm.full[i]);
             }
             asm volatile("griddepcontrol.wait;" ::: "memory");
+            *static_cast<volatile int *>(&sm.started) = 1;
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             // token rows past n_tok are outside the tensor map and arrive as zeros
             for (int i = 0; i < pre; ++i) tma_load_3d(sm.ring + i * stage_bytes, &x_map, 0, tok0, k_base + i * kb, &sm.full[i]);
@@ -516,7 +520,7 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             // D = f32, A = B = f16, both K-major, N = n_box, M = 128
             const uint32_t idesc = (1u << 4) | ((static_cast<uint32_t>(a.n_box) >> 3) << 17) | ((128u >> 4) << 24);
             for (int i = 0, st = 0, round = 0; i < n_k; ++i) {
-                if (!mbar_wait_bounded(&sm.full[st], round & 1u, &sm.abort_flag)) break;
+                if (!mbar_wait_bounded(&sm.full[st], round & 1u, &sm.abort_flag, &sm.started)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t xs = smem_u32(sm.ring + st * stage_bytes), wsm = xs + x_bytes;
 #pragma unroll 1

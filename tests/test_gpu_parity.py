@@ -373,6 +373,36 @@ def test_fused_splitkv_step_four_ranks_on_one_device():
     arena.close()
 
 
+@pytest.mark.parametrize("n_out", [4096, 96])   # features on the M side, k split over a cluster; tokens on the M side
+def test_linear_behind_a_kernel_that_waits_longer_than_a_bounded_wait(n_out):
+    """A split-KV step releases its successor before it waits for its peers; here the only peer stays silent for the 1.5 s that the
+    step was given.  The Linear behind it, which comes up meanwhile, counts none of that against its own bounded waits."""
+    from chatglm_cpp_b200 import _lib
+    A = _A()
+    H, G, D, P, n_tok, n_in = 32, 2, 128, 300, 4, 1024
+    desc = make_desc(H, G, D, 512)
+    arena, ws = A.KVArena(desc, 1), A.Workspace(desc, 1, 1)
+    bufs = [A.SplitKVExchange.new_buffer(2, H, D) for _ in range(2)]
+    rank0 = A.SplitKVExchange(bufs, 0, H, D)
+    arr = (_lib.AttnSeq * 1)()
+    qkv = torch.randn(1, qkv_width(desc, False), device="cuda")
+    A.fill_seq(arr[0], desc, A.SeqCall(qkv=qkv, slot=0, n_past=P, kv_local=P, flags=A.SEQ_USE_KV_LOCAL), False)
+    L = _lib.lib()
+    own = A.Workspace(desc, 1, 1)
+    x, w = torch.randn(n_tok, n_in, device="cuda").half(), torch.randn(n_out, n_in, device="cuda").half()
+    out, out_step = torch.empty(n_tok, n_out, device="cuda"), torch.zeros(H * D, device="cuda")
+    torch.cuda.synchronize()
+    rank0.step(arena, ws, arr, out_step, combine=True, timeout_us=1500000)
+    _lib.check(L.cglm_linear_forward(x.data_ptr(), n_tok, n_in, w.data_ptr(), n_out, None, out.data_ptr(), 0, own.ptr, own.bytes,
+                                     torch.cuda.current_stream().cuda_stream), "cglm_linear_forward")
+    torch.cuda.synchronize()
+    assert ws.status() == _lib.ERR_TIMEOUT   # the step's own bound
+    assert own.status() == 0
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((out.double() - want).abs() <= 8 * 2.0 ** -24 * n_in ** 0.5 * size).all()
+    arena.close()
+
+
 def test_fused_splitkv_step_single_rank_equals_plain_decode():
     """One rank: the step degenerates to decode + normalisation and must agree with cglm_attn_forward; a sequence short
     enough that one thread block holds a whole kv head takes the other publication path."""
