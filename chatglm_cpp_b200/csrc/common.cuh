@@ -60,9 +60,13 @@ struct AttnShape {
 };
 
 // ---- bounded waiting --------------------------------------------------------------------------------
-// Every device-side wait in this library gives up after kSpinLimit polls, records CGLM_ERR_TIMEOUT in the
-// workspace status word and lets the kernel run to its end with invalid results instead of hanging.
-constexpr unsigned int kSpinLimit = 1u << 22;
+// Every device-side wait in this library gives up after a time (kSpinLimit bounds the loops around them), records
+// CGLM_ERR_TIMEOUT in the workspace status word and lets the kernel run to its end with invalid results instead of hanging.
+constexpr unsigned int kSpinLimit = 1u << 25;
+constexpr unsigned long long kGateLimitNs = 4000000000ull;    // for a word that a copy engine writes (DecodeTable::gate)
+constexpr unsigned long long kWaitLimitNs = 10000000000ull;   // for an mbarrier
+// the warps of a launch that wait for its q wait while one of them waits for the two gates in turn
+static_assert(kWaitLimitNs > 2 * kGateLimitNs, "a gate's bound must run out before that of the waits behind it");
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -115,7 +119,6 @@ __device__ __forceinline__ bool mbar_try_wait_for(uint64_t *bar, uint32_t parity
 // Returns false when the wait ran out (or this one is not met and an earlier wait of this CTA ran out): the caller carries
 // on without touching the barrier again.  *abort_flag lives in shared memory.  A waiting warp suspends in the barrier instead
 // of polling (polls take issue slots from the warps that work), so the wait is bounded by time: at most kWaitLimitNs.
-constexpr unsigned long long kWaitLimitNs = 1000000000ull;
 // started: for a wait that may begin before this grid's dependency wait, a word that is set once the kernel in front has
 // completed; the time until then does not count.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort_flag, volatile int *started = nullptr) {

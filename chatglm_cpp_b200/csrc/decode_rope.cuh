@@ -72,10 +72,14 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
 }
 // Polls a word that a copy engine writes, with a bound; false when it ran out.
 __device__ __forceinline__ bool wait_gate(const unsigned int *word, unsigned int value, volatile int *abort_flag) {
+    unsigned long long t0 = 0, now;
     for (unsigned int spin = 0; spin < kSpinLimit && !*abort_flag; ++spin) {
         unsigned int v;
         asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
         if (v == value) return true;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (t0 == 0) t0 = now;
+        if (now - t0 > kGateLimitNs) break;
         __nanosleep(200);
     }
     return false;
