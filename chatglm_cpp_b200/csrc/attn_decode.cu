@@ -626,7 +626,7 @@ __device__ __forceinline__ void merge_staged(const DeliverArgs *da, const Global
                     for (int x = kMergeSlots; x < n; ++x) bulk_load(slots + (x - kMergeSlots) * kDecodePartialFloats, g(k0 + x), kBytes, &bars[1]);
                 }
             }
-            ok = mbar_wait_bounded(&bars[1], use1 & 1u, da->abort_flag);
+            ok = mbar_wait_bounded(&bars[1], use1 & 1u, da->abort_flag) && ok;
         }
         if (ok && r < R) merge_four(st, k0 + i, k1, r, d0, src);
     }
