@@ -476,8 +476,8 @@ constexpr int kMergeFan = kDecodeMergeFan;
 // begins inside the group (slot 1).
 __device__ __forceinline__ int group_slot(long long grp, long long b0) { return b0 < grp * kMergeFan ? 0 : 1; }
 
-// 16 dims of one q row merged over sources k0..k1 in one pass with a running maximum, four sources at a time.  Sources are CTA partials (level 0) or group partials (level 1): source k sits at base + 2k slots (stride 2),
-// except that source k_first uses its second slot when first_slot is 1 (the CTA or group in which the item begins
+// 16 dims of one q row merged over sources k0..k1 in one pass with a running maximum, four sources at a time.  Sources are CTA
+// partials (level 0) or group partials (level 1): source k sits at base + 2k slots (stride 2), except that source k_first uses its second slot when first_slot is 1 (the CTA or group in which the item begins
 // holds the end of the previous item in its first slot).  The fused split-KV step merges the ranks' copies of a kv
 // head with the same routine: source = rank, stride = kv heads per rank slot.  Every caller goes through merge_four with the
 // same source order and explicit roundings, so the result does not depend on which CTA or warp completes the item.
@@ -591,10 +591,6 @@ __device__ __forceinline__ void merge_row_chunk(const float *base, int stride, l
 }
 // The same sums by the four consumer warps together, thread t for row t / 8 and dims 16 (t % 8) ..: the parts come into the
 // tile ring by bulk copies.  use, use1: how often the two barriers have been used before (their phases).
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
-                 "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void merge_staged(const DeliverArgs *da, const GlobalParts &g, long long k0, long long k1, float *dst,
                                              int dst_kind, int t, int R, uint32_t use, uint32_t use1) {
     constexpr uint32_t kBytes = kDecodePartialFloats * 4;
@@ -1389,11 +1385,13 @@ cudaError_t launch_decode(const LaunchCtx &cx, const DecodeTableDyn &tab, bool n
     // B200: 64 sequences (9.3 k tiles) 61.8 us per launch with 259 CTAs, 63.3 with 228, 68.3 with 148, 62.7 with 296;
     // 32 sequences (4.7 k tiles) 39.9 us with 259 against 42.2 with 148; the MHA shape 34.9 us with 200 against 37.9
     // with 148; 16 and 8 sequences and the one long sequence do not care between 96 and 228.
-    // A launch with fewer tiles than SMs (batch-1 decode of a short context) is all latency, and what costs is the number
-    // of parts an item is delivered in: measured on one 512-token sequence (2 items of 9 tiles), 18 CTAs of one tile
-    // 11.0 us per launch, 9 CTAs of two tiles (spans that straddle the items) 17.2 us, 6 CTAs of three tiles 9.6 us, 2
-    // CTAs of nine tiles 11.4 us.  Such a launch is cut into at most four parts per item (one batch of the merge) of
-    // about three tiles each; with items of equal length the spans then end where the items do.
+    // A launch with fewer tiles than SMs is all latency, and what costs is the number of parts an item is delivered in.  Such a
+    // launch is cut into at most four parts per item (one batch of the merge) of about three tiles each; with items of equal
+    // length the spans then end where the items do.  The launches for which that was measured (one 512-token sequence, 2
+    // items of 9 tiles: 18 CTAs of one tile 11.0 us, 9 of two, straddling the items, 17.2, 6 of three 9.6) run in clusters
+    // now.  What still comes here is many items of a tile or two, and a few items just past the clusters' line, for which four
+    // parts are too few: 2 items of 65 to 73 tiles 17.1 to 18.2 us with the 8 CTAs of this rule, 14.1 to 14.4 with 16 to 32,
+    // 17.3 to 17.8 with 148.
     const long long lo_ctas = cx.n_sm, hi_ctas = 7LL * cx.n_sm / 4;
     long long want = total_tiles / 18;
     want = want < lo_ctas ? lo_ctas : (want > hi_ctas ? hi_ctas : want);

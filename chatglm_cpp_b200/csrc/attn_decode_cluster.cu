@@ -31,7 +31,7 @@ constexpr int kQStride = 136;         // halfs per q row (272 B): the eight-byte
 // Asked for instead of what ClusterSmem takes: thread blocks of one launch then spread over the SMs (two would not fit one),
 // every kernel of the step runs with the same split of an SM's memory, without which they could not share SMs at all, and a
 // thread block of the Linear kernels (kFmSplitSmem) still fits beside.
-constexpr int kSmemBytes = 117248;
+constexpr int kSmemBytes = kDecodeClusterSmem;
 constexpr int kRoundsAhead = 4;       // rounds of the cluster asked for in L2 before the wait
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -55,10 +55,6 @@ struct __align__(16) ClusterSmem {
     int abort_flag;
 };
 
-__device__ __forceinline__ void cluster_sync() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ uint32_t peer_addr(const void *p, int rank) {
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));

@@ -59,7 +59,7 @@ constexpr uint32_t kIdescS = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24
 constexpr uint32_t kIdescO = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
 struct __align__(1024) PrefillSmem {
-    uint8_t q[2][kTileBytes];         // A of QK^T per group: [2 d-halves][128 rows][64 d]; staging of the output at the end
+    uint8_t q[2][kTileBytes];         // A of QK^T per group: [2 d-halves][128 rows][64 d]
     uint8_t kv[kStages][kTileBytes];  // K tile [2 d-halves][128 tokens][64 d] or V^T tile [2 token-halves][128 d][64 tokens]
     uint64_t kv_full[kStages];        // TMA -> MMA: tile landed
     uint64_t kv_empty[kStages];       // tensor core -> TMA: tile has been read by both groups' MMAs
@@ -436,11 +436,6 @@ __device__ __forceinline__ void stage_q(const PrefillSeq &ps, const AttnShape &s
             *reinterpret_cast<uint4 *>(at(w) + (hl >> 3) * kHalfBytes + r * 128 + (((hl & 7) ^ (r & 7)) << 4)) = pack_half8(y);
         }
     }
-}
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
-                 "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
 }
 // 32 bytes of one thread to global memory: one full sector per lane
 __device__ __forceinline__ void st_sector(void *p, const uint32_t (&v)[8], int align) {

@@ -149,7 +149,7 @@ struct WsLayout {
 WsLayout ws_layout(const cglm_attn_desc &d, int n_sm, int n_seq, long long n_tokens, size_t prefill_bytes = 0) {
     WsLayout w;
     size_t off = sizeof(WsHeader);
-    // q tiles of long prompts (PrefillTable), the room that every workspace also offers the Linears
+    // q tiles of long prompts
     off = align_up(off + kLinearScratchBytes, 256);
     w.counters = off;
     off = align_up(off + sizeof(int) * kDecodeMaxSeqPerLaunch * static_cast<size_t>(d.n_kv_head), 256);

@@ -163,6 +163,18 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
+// Untiled copy of this GPU's own memory into shared memory; both addresses and the size multiples of 16 bytes.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
+                 "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+// every thread of the cluster, and its memory operations
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ---- warp-level tensor-core pieces for the decode kernel ---------------------------------------------
 __device__ __forceinline__ void ldmatrix_x4(uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3, uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -301,7 +313,7 @@ struct LaunchCtx {
     float *partials;             // decode split partials: 2 slots per CTA
     float *gpartials;            // decode group partials: 2 slots per group of 16 CTAs
     float *q_stage;              // generic path: roped, scaled q f32 [tokens][H][D]
-    uint8_t *q_tiles;            // prompt attention: two f16 q tiles per CTA (the Linear kernels' scratch region)
+    uint8_t *q_tiles;            // prompt attention: two f16 q tiles per CTA (kLinearScratchBytes)
     const CUtensorMap *k_map;    // host copies of the arena's tensor maps (passed by value to kernels)
     const CUtensorMap *v_map;
     const float2 *rope_tab;      // arena's angle table: [rope_tab_len positions][32 ladder steps] (cos, sin); may be null
@@ -375,6 +387,7 @@ cudaError_t launch_decode(const LaunchCtx &cx, const DecodeTableDyn &tab, bool n
                           const XchgDev *xchg = nullptr);
 // the same for a small launch, one cluster of n_cta (2, 4, 8) thread blocks per (sequence, kv head)
 constexpr int kDecodeClusterMaxSeq = 64;
+constexpr int kDecodeClusterSmem = 117248;   // shared memory of such a thread block
 cudaError_t launch_decode_cluster(const LaunchCtx &cx, const DecodeTable &tab, int n_cta);
 // how many clusters of n_cta such thread blocks the (current) device runs at once; 0 when that cannot be told
 int decode_cluster_resident(int device, int n_cta);
@@ -389,7 +402,7 @@ inline bool decode_rows_aligned(const float *q, const float *k, const float *v, 
 // tcgen05 path of prompts (n_past == 0, head_dim 128): what the two launches know about up to kPrefillMaxSeq of them, passed by
 // value.  A sequence's V^T tensor map ends at its attended length.
 constexpr int kPrefillMaxSeq = 8;
-constexpr int kPrefillMaxCtas = 148;   // x 64 KiB of q tiles: what the Linear kernels' scratch holds
+constexpr int kPrefillMaxCtas = 148;   // x 64 KiB of q tiles: kLinearScratchBytes
 enum { kPrefillSingle = 0, kPrefillPairHeads = 1, kPrefillPairTiles = 2 };   // q tiles per CTA, and which two
 struct PrefillSeq {
     SeqDev sq;
@@ -426,9 +439,11 @@ cudaError_t launch_qkv_linear(const LaunchCtx &cx, const CUtensorMap &x_map, con
 cudaError_t launch_linear_plain(int device, cudaStream_t stream, WsHeader *hdr, const CUtensorMap &x_map, const CUtensorMap &w_map,
                                 int n_tok, int K, int n_feat, int kb, const float *bias, void *out, bool out_f16);
 // The Linear with the output features on the M side of the MMA (n_feat a multiple of 128): k split over the CTAs of a
-// cluster per 128-feature tile (two CTAs or four; up to 60 tiles).
+// cluster per 128-feature tile, two CTAs or four, up to 60 tiles.  Two CTAs for each of 61 to 74 tiles would fit the SMs too but
+// are slower than one (k 4096, 1 / 128 tokens: 61 tiles 18.2 -> 18.6 / 23.6 -> 25.5 us, 74 tiles 18.9 -> 21.2 / 24.6 -> 27.7).
 constexpr int kLinearFmMaxSplitTiles = 60;
-// what a workspace holds for the Linears (cglm_linear_workspace_bytes); a call with less runs with the tokens on the M side
+// Behind the header of every workspace: the q tiles of prompts.  The Linears use none of it; a call whose workspace lacks it
+// runs with the tokens on the M side, which is what cglm_linear_forward documents, and so keeps the order of its sums.
 constexpr size_t kLinearScratchBytes = static_cast<size_t>(148) * 128 * 128 * sizeof(float);   // 148 CTAs x [128 tokens][128 features]
 struct LinearFmPlan {
     int n_box, tiles, token_tiles, ksplit, blocks_per_cta, kb, n_stages, tmem_cols;

@@ -307,16 +307,17 @@ qkv_linear_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
 // dependency wait.
 //
 // Measured (per replay of a 28-layer step of one 512-token chat, every layer's own weights, with decode_cluster_kernel between
-// the Linears): with the partial sums through L2, a counter and all of an SM's shared memory 1020 us, as it is now 815 us; 64
-// sequences x 4 layers 371 -> 365 us.
+// the Linears): with the partial sums through L2, a counter and all of an SM's shared memory 1020 us, as it is now 800 us; 64
+// sequences x 4 layers 371 -> 360 us.
 constexpr int kFmFeat = 128;                 // M of the MMA: output features per CTA
 constexpr int kFmWBytes = kFmFeat * 128;     // W tile of one 64-k block: [128 features][64 k] f16
 constexpr int kFmMaxStages = 8;
 // (token, 4 features) items a thread has in flight in the finishing pass: up to 64 tokens are one batch
 constexpr int fm_batch(int ksplit) { return ksplit == 4 ? 3 : 6; }
-// Shared memory of a CTA of a split launch: two such CTAs, or one beside a CTA of the decode kernel (at most this much as
-// well), fit the 228 KiB of an SM with 1 KiB reserved for each.
+// Shared memory of a CTA of a split launch: two such CTAs, or one beside a CTA of decode_cluster_kernel, fit the 228 KiB of an
+// SM with 1 KiB reserved for each.
 constexpr int kFmSplitSmem = 112640;
+static_assert(2 * (kFmSplitSmem + 1024) <= 233472 && kFmSplitSmem + kDecodeClusterSmem + 2048 <= 233472, "two thread blocks per SM");
 // The requests into L2 leave this much after the ring's: at once they stand in front of what the previous kernel still has to
 // load (829 us per step with no delay, 824 / 815 / 813 with 1 / 2 / 3.5 us).
 constexpr unsigned int kFmPrefetchDelayNs = 2000;
@@ -350,10 +351,6 @@ struct FmArgs {
     const float2 *rope_tab;
     int rope_tab_len;
 };
-
-__device__ __forceinline__ void cluster_sync() {   // every thread of the cluster, and its memory operations
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 template <bool kPlain>
 __device__ __forceinline__ void fm_finish_item(const FmArgs &a, const QkvTable &tab, const AttnShape &sh, int f0, int tok, int q, float4 v) {
@@ -562,7 +559,6 @@ linear_fm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             for (int j = 0; j < 16; ++j) dump[(c + j) * kFmFeat + tid] = __uint_as_float(r[j]);   // rows < n_box: inside the ring
         }
     }
-    __syncwarp();   // the cluster barrier below wants whole warps
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     // every thread that writes an output has seen the previous kernel complete
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -59,12 +59,12 @@ def test_host_only_entry_points_without_a_gpu():
 
 
 def test_linear_kernel_plan_stays_inside_its_buffers():
-    """cglm_linear_kernel_plan over a grid of shapes: what the launcher would ask of shared memory, tensor memory, the
-    workspace scratch and the tile counters stays inside what exists (a plan outside them would fault on the device)."""
+    """cglm_linear_kernel_plan over a grid of shapes: what the launcher would ask of shared memory and tensor memory stays inside
+    what exists (a plan outside them would fault on the device): a thread block's ring or its sums [tokens][128] in the ring's
+    place, of a split launch in half an SM, so that the thread blocks of all its clusters run at once."""
     from chatglm_cpp_b200 import _lib
     L = _lib.lib()
-    scratch = L.cglm_linear_workspace_bytes() - 256
-    smem_per_cta = 232448
+    smem_per_cta, smem_per_sm, smem_split, reserved = 232448, 233472, 112640, 1024
     taken = 0
     for n_sm in (148, 132, 64):
         for n_tok in (1, 7, 8, 16, 17, 32, 33, 64, 100, 128, 129, 200, 256, 1000, 1024, 4096, 8192):
@@ -86,7 +86,9 @@ def test_linear_kernel_plan_stays_inside_its_buffers():
                     if ksplit > 1:
                         ctas = tiles * ttiles * ksplit
                         assert ctas <= n_sm and tiles * ttiles <= 60, what
-                        assert ctas * n_box * 128 * 4 <= scratch, what
+                        asked = 2048 + max(stages * stage_bytes, n_box * 128 * 4)   # what the launch asks for
+                        assert asked <= smem_split and 2 * (asked + reserved) <= smem_per_sm, what
+                        assert stages >= min(3, blocks // kb) or kb == 1, what       # boxes in flight
                     else:
                         assert stages * stage_bytes >= n_box * 128 * 4, what       # the sums pass through the ring
     assert taken > 500

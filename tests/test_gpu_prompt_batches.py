@@ -145,3 +145,39 @@ def test_prompt_rows_whose_first_scores_are_minus_infinity(H, G, S):
     want = torch.einsum("sgrt,gdt->sgrd", torch.softmax(sc, -1), v).reshape(S - N, H * 128)
     assert_out_close(out[N:].cpu().numpy(), want.numpy().astype(np.float32), f"{S} tokens")
     arena.close()
+
+
+@pytest.mark.parametrize("H,G,rope,mask", [(6, 2, O.ROPE_CHATGLM2, O.MASK_CAUSAL), (4, 4, O.ROPE_CHATGLM, O.MASK_CHATGLM)])
+@pytest.mark.parametrize("offset", [4, 8, 16])   # f16 output rows on 8-, 16- and 32-byte boundaries only
+def test_prompts_with_ids_of_their_own_and_f16_outputs(H, G, rope, mask, offset):
+    """Three prompts in one call: ids derived, ids of the caller's that go beyond the cache's angle table, and the derived ids passed
+    explicitly.  f16 in and out, the outputs at every alignment of their rows that the store distinguishes."""
+    from chatglm_cpp_b200 import attention as A
+    inter = rope == O.ROPE_CHATGLM
+    desc = make_desc(H, G, 128, 328, 0, rope, 10000.0, mask)
+    rng = np.random.default_rng(offset)
+    lens, width, cfg = [190, 130, 257], qkv_width(desc, inter), oracle_cfg(desc, "f32")
+    arena, ws = A.KVArena(desc, 3), A.Workspace(desc, 3, max(lens))
+    calls, inputs, ids = [], [], []
+    for i, S in enumerate(lens):
+        x = rng.standard_normal((S, width)).astype(np.float16)
+        own = O.position_ids(cfg, S, 0, S).astype(np.int32)
+        if i == 1:
+            own = rng.integers(0, 2000, own.shape).astype(np.int32)
+        out = torch.zeros(offset + S * H * 128, device="cuda", dtype=torch.float16)[offset:].view(S, H * 128)
+        assert out.data_ptr() % (2 * offset) == 0 and (offset == 16 or out.data_ptr() % (4 * offset) != 0)
+        calls.append(A.SeqCall(qkv=torch.from_numpy(x).cuda(), slot=i, n_past=0, n_ctx=S, out=out,
+                               position_ids=torch.from_numpy(own).cuda() if i else None))
+        inputs.append(x.astype(np.float32))
+        ids.append(own)
+    A.forward_batch(arena, ws, calls, inter)
+    torch.cuda.synchronize()
+    assert ws.status() == 0
+    for i, S in enumerate(lens):
+        k, v = (np.zeros((G, 328, 128), np.uint16), np.zeros((G, 128, 328), np.uint16))
+        want = O.attn_forward(cfg, inputs[i], inter, k, v, 0, n_ctx=S, ids=ids[i])
+        assert_out_close(calls[i].out.float().cpu().numpy(), want.astype(np.float16).astype(np.float32), f"prompt {i} of {S} tokens")
+        gk, gv = download_cache(arena, i)
+        np.testing.assert_array_equal(gk, k)
+        np.testing.assert_array_equal(gv, v)
+    arena.close()
