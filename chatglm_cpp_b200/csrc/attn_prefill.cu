@@ -16,8 +16,9 @@
 //   MMA warps      one per group.  Q K^T of step t + 1 runs while the softmax works on step t, P V of t follows it.  tcgen05.mma
 //                  of one thread execute in order: a group that sees its scores of step t knows that P V of t - 2 has landed.
 //   q warps        stage the q tiles of the CTA's next unit (CTAs are persistent; units are dealt longest first).
-// Measured (B200, 32 q heads, 2 kv heads, causal, f16 activations): an 8192-token prompt alone 499 us, 563 us back to back
-// under the power cap (977 TFLOP/s of useful work), against 795 us with one q tile per CTA, probabilities through shared memory and q staged through HBM by a kernel of its own.
+// Measured (B200, 32 q heads, 2 kv heads, causal): an 8192-token prompt alone 491 us, 555 us back to back under the power cap
+// (990 TFLOP/s of useful work), against 795 us with one q tile per CTA, probabilities through shared memory and q staged
+// through HBM by a kernel of its own.
 // A step takes about 1600 cycles; taking a quarter of the exponentials off their unit (a polynomial on the FMA pipe) made it
 // slower, because what the softmax warps issue delays the MMA warps, which need about a tenth of the issue slots.
 // O stays in tensor memory across KV tiles; a row's O is rescaled there only when its running maximum grows by more than
