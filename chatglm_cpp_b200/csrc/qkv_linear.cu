@@ -700,8 +700,15 @@ bool linear_fm_plan(int n_tok, int K, int n_feat, int n_sm, LinearFmPlan *p) {
     }
     p->blocks_per_cta = K / kKStep / p->ksplit;
     // an unsplit launch has an SM to itself and does best with large boxes and two stages; a split one is smaller and keeps
-    // three boxes in flight (its sums are 64 KiB at most, less than any ring of three)
-    const int ring = (p->ksplit > 1 ? kFmSplitSmem : kSmemPerCta) - 2048;
+    // three boxes in flight (its sums are 64 KiB at most, less than any ring of three).  A split launch with a long way to go
+    // whose boxes are so large that only three single blocks fit takes the SM to itself as well: what it keeps in flight then
+    // counts for more than what it had before the dependency wait (k 13696 to 4096 features, 96 / 128 tokens: 56.9 / 58.3 us with
+    // the small ring, 50.7 / 51.9 with the whole SM; up to 80 tokens, four stages and more, the small one does).  32 clusters of four
+    // such thread blocks are resident on every B200, more need not be.
+    const int stage1 = p->n_box * 128 + kFmWBytes;
+    const bool whole_sm = p->ksplit == 1 || ((kFmSplitSmem - 2048) / stage1 <= 3 && p->blocks_per_cta > 32 &&
+                                             (p->ksplit == 2 || tiles * ttiles <= 32));
+    const int ring = (whole_sm ? kSmemPerCta : kFmSplitSmem) - 2048;
     p->kb = 1;
     for (int kb = 4; kb > 1; kb >>= 1) {
         if (p->blocks_per_cta % kb == 0 && ring / (kb * (p->n_box * 128 + kFmWBytes)) >= (p->ksplit > 1 ? 3 : 2)) {

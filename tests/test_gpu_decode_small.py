@@ -137,10 +137,11 @@ def test_merged_parts_are_those_of_the_launch(G, P):
     arena.close()
 
 
-@pytest.mark.parametrize("n_tok,n_in,n_out", [(128, 256, 128), (128, 512, 4096), (33, 4096, 4608), (1, 128, 128), (17, 4160, 256)])
+@pytest.mark.parametrize("n_tok,n_in,n_out", [(128, 256, 128), (128, 512, 4096), (33, 4096, 4608), (1, 128, 128), (17, 4160, 256),
+                                              (100, 8576, 256), (128, 8576, 4608), (128, 8448, 4096)])   # a whole SM each
 def test_linear_k_split_over_a_cluster(n_tok, n_in, n_out):
     """Fewer weight blocks than the sums need room, one block per thread block, token counts that no CTA's share divides, a k that
-    four does and does not split evenly.  Bound: f32 sums of n_in products of f16 values, 2^-24 * sqrt(n_in) of the sum of their
+    four does and does not split evenly, long slices of k by clusters of two and of four.  Bound: f32 sums of n_in products of f16 values, 2^-24 * sqrt(n_in) of the sum of their
     sizes with a factor of 8."""
     from chatglm_cpp_b200 import _lib
     gen = torch.Generator(device="cuda")
